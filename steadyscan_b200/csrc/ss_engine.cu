@@ -2385,13 +2385,72 @@ static void fe_blur(const void* in, double* w1, double* w2, int h, int w, int n,
   k_blur_pass<double, 1><<<grid, 256, 0, s>>>(w1, w2, h, w, pw, tx, rx);
 }
 
+// Recognises a block map of whole lines (k_block_rows): fills start (nb + 1 cropped rows) and returns
+// the most lines of a block, or 0 for any other map. Every entry is checked.
+static int row_blocks(const int* gather, int hb, int nb, int hc, int wc, std::vector<int>& start) {
+  start.assign((size_t)nb + 1, 0);
+  int kmax = 0;
+  for (int b = 0; b < nb; b++) {
+    const int* g = gather + (size_t)b * hb;
+    const int s = g[0];
+    if (s < 0 || s >= hc || (b > 0 && s != start[b])) return 0;
+    int k = 1;
+    while (k < hb && k <= kRowMaxLines && s + k < hc && g[k] == s + k) k++;
+    if (k > kRowMaxLines || (int64_t)k * wc > hb) return 0;
+    const int m = k * wc;
+    int bad = 0;
+    for (int r = k; r < m; r++) bad |= (g[r] - g[r - k]) ^ hc;
+    for (int r = m; r < hb; r++) bad |= g[r] ^ -1;
+    if (bad) return 0;
+    start[b] = s;
+    start[b + 1] = s + k;
+    kmax = std::max(kmax, k);
+  }
+  return kmax;
+}
+
+// A block map on the device: the row starts of a map of whole lines (kmax > 0), else its entries.
+struct BlockMap {
+  const int* d = nullptr;
+  int kmax = 0, bt = 1;        // most lines of a block; blocks of a tile
+  std::vector<int> start;      // kmax > 0: nb + 1 row starts
+};
+
+template <class InT, class OutT>
+static void fe_gather_to(const InT* in, OutT* out, int h, int w, int n, int r0, int c0, int hc, int wc,
+                         const BlockMap& map, int hb, int nb, cudaStream_t s) {
+  if (!map.kmax) {
+    k_block_gather<InT, OutT><<<148 * 8, 256, 0, s>>>(in, out, h, w, n, r0, c0, hc, map.d, hb, nb);
+    return;
+  }
+  constexpr int kVec = 16 / sizeof(InT);
+  bool vec = (size_t)h % kVec == 0 && reinterpret_cast<uintptr_t>(in) % 16 == 0;
+  for (int b = 0; b < nb && vec; b += map.bt) vec = (r0 + map.start[b]) % kVec == 0;
+  constexpr int kOut = 16 / sizeof(OutT);
+  const bool wide = hb % kOut == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0;
+  const dim3 grid((nb + map.bt - 1) / map.bt, (wc + kRowTile - 1) / kRowTile, n);
+  const int slots = kRowTile * map.kmax / (wide ? kOut : 1);
+  const unsigned inv = (unsigned)((0x100000000ull + slots - 1) / slots);
+#define SS_ROWS(VE, VO, K) \
+  k_block_rows<InT, OutT, VE, VO, K><<<grid, 256, 0, s>>>(in, out, h, w, r0, c0, wc, map.d, hb, nb, map.bt, slots, inv)
+  const int k = (map.start[nb] - map.start[0]) == nb * map.kmax ? map.kmax : 0;  // every block has k lines
+  if (vec && wide && k == 1) SS_ROWS(kVec, kOut, 1);
+  else if (vec && wide && k == 2) SS_ROWS(kVec, kOut, 2);
+  else if (vec && wide && k == 4) SS_ROWS(kVec, kOut, 4);
+  else if (vec && wide) SS_ROWS(kVec, kOut, 0);
+  else if (vec) SS_ROWS(kVec, 1, 0);
+  else if (wide) SS_ROWS(1, kOut, 0);
+  else SS_ROWS(1, 1, 0);
+#undef SS_ROWS
+}
+
 template <class InT>
-static void fe_gather(const void* in, int out_dt, void* out, int h, int w, int n, int r0, int c0, int hc,
-                      const int* gather, int hb, int nb, cudaStream_t s) {
-  const int g = 148 * 8;
-  if (out_dt == SS_F64) k_block_gather<InT, double><<<g, 256, 0, s>>>(in, (double*)out, h, w, n, r0, c0, hc, gather, hb, nb);
-  else if (out_dt == SS_F32) k_block_gather<InT, float><<<g, 256, 0, s>>>(in, (float*)out, h, w, n, r0, c0, hc, gather, hb, nb);
-  else k_block_gather<InT, uint16_t><<<g, 256, 0, s>>>(in, (uint16_t*)out, h, w, n, r0, c0, hc, gather, hb, nb);
+static void fe_gather(const void* in, int out_dt, void* out, int h, int w, int n, int r0, int c0, int hc, int wc,
+                      const BlockMap& map, int hb, int nb, cudaStream_t s) {
+  const InT* x = static_cast<const InT*>(in);
+  if (out_dt == SS_F64) fe_gather_to(x, (double*)out, h, w, n, r0, c0, hc, wc, map, hb, nb, s);
+  else if (out_dt == SS_F32) fe_gather_to(x, (float*)out, h, w, n, r0, c0, hc, wc, map, hb, nb, s);
+  else fe_gather_to(x, (uint16_t*)out, h, w, n, r0, c0, hc, wc, map, hb, nb, s);
 }
 
 int prepare_frames(const ss_prep_frames* p) {
@@ -2407,9 +2466,20 @@ int prepare_frames(const ss_prep_frames* p) {
   const int64_t hc = h - cr[2] - cr[3], wc = w - cr[0] - cr[1];
   const int hb = p->block_h, nbk = p->n_blocks;
   if (!p->gather || hb < 1 || nbk < 1) return fail(SS_ERR_INVALID_ARGUMENT, "prepare_frames: empty block map");
-  for (int64_t i = 0; i < (int64_t)hb * nbk; i++)
-    if (p->gather[i] < -1 || p->gather[i] >= hc * wc)
+  BlockMap map;
+  // the tiles' frame index is the grid's z extent and the column tiles its y extent
+  if (hc <= INT_MAX && wc <= (int64_t)65535 * kRowTile)
+    map.kmax = row_blocks(p->gather, hb, nbk, (int)hc, (int)wc, map.start);
+  if (!map.kmax) {
+    int lo = 0;
+    int64_t hi = -1;
+    for (int64_t i = 0; i < (int64_t)hb * nbk; i++) {
+      lo = std::min(lo, p->gather[i]);
+      hi = std::max<int64_t>(hi, p->gather[i]);
+    }
+    if (lo < -1 || hi >= hc * wc)
       return fail(SS_ERR_INVALID_ARGUMENT, "prepare_frames: block map index outside the cropped frame");
+  }
   const ss_matrix& o = p->out;
   if (o.location != SS_DEVICE || !o.data || o.rows != hb || o.cols != (int64_t)nbk * n)
     return fail(SS_ERR_INVALID_ARGUMENT, "prepare_frames: out must be block_h x (n_blocks * n_frames) on the device");
@@ -2446,7 +2516,8 @@ int prepare_frames(const ss_prep_frames* p) {
   CallMem m;
   SS_CK(cudaStreamCreateWithFlags(&m.s, cudaStreamNonBlocking));
   cudaStream_t s = m.s;
-  int* d_gather = m.take<int>((size_t)hb * nbk);
+  const size_t map_n = map.kmax ? map.start.size() : (size_t)hb * nbk;
+  int* d_gather = m.take<int>(map_n);
   double* d_taps = blur ? m.take<double>(ty.size() + tx.size()) : nullptr;
   void* d_raw = p->frames.location == SS_HOST ? m.take<char>(fsz * npx * chunk) : nullptr;
   double* w1 = (blur || med) ? m.take<double>(npx * chunk) : nullptr;
@@ -2455,7 +2526,17 @@ int prepare_frames(const ss_prep_frames* p) {
   if (!d_gather || (blur && !d_taps) || (p->frames.location == SS_HOST && !d_raw) || ((blur || med) && !w1) ||
       (blur && !w2) || (med && !d_med))
     return fail(SS_ERR_OUT_OF_MEMORY, "prepare_frames: work memory");
-  SS_CK(cudaMemcpyAsync(d_gather, p->gather, (size_t)hb * nbk * sizeof(int), cudaMemcpyHostToDevice, s));
+  SS_CK(cudaMemcpyAsync(d_gather, map.kmax ? map.start.data() : p->gather, map_n * sizeof(int), cudaMemcpyHostToDevice,
+                        s));
+  map.d = d_gather;
+  if (map.kmax) {  // blocks of a tile: a multiple of 8 rows where the lines per block allow it (aligned reads)
+    map.bt = std::max(1, kRowTile / map.kmax);
+    for (int t = map.bt; t > 1; t--)
+      if ((t * map.kmax) % 8 == 0) {
+        map.bt = t;
+        break;
+      }
+  }
   if (blur) {
     SS_CK(cudaMemcpyAsync(d_taps, ty.data(), ty.size() * 8, cudaMemcpyHostToDevice, s));
     SS_CK(cudaMemcpyAsync(d_taps + ty.size(), tx.data(), tx.size() * 8, cudaMemcpyHostToDevice, s));
@@ -2494,10 +2575,10 @@ int prepare_frames(const ss_prep_frames* p) {
       k_frame_divide<<<g, 256, 0, s>>>(x, npx, npx * c, d_med);
     }
     void* dst = static_cast<char*>(const_cast<void*>(o.data)) + osz * (size_t)hb * nbk * f0;
-    if (cur_dt == SS_F64) fe_gather<double>(cur, o.dtype, dst, (int)h, (int)w, c, r0, c0, (int)hc, d_gather, hb, nbk, s);
-    else if (cur_dt == SS_F32) fe_gather<float>(cur, o.dtype, dst, (int)h, (int)w, c, r0, c0, (int)hc, d_gather, hb, nbk, s);
-    else if (cur_dt == SS_U16) fe_gather<uint16_t>(cur, o.dtype, dst, (int)h, (int)w, c, r0, c0, (int)hc, d_gather, hb, nbk, s);
-    else fe_gather<__half>(cur, o.dtype, dst, (int)h, (int)w, c, r0, c0, (int)hc, d_gather, hb, nbk, s);
+    if (cur_dt == SS_F64) fe_gather<double>(cur, o.dtype, dst, (int)h, (int)w, c, r0, c0, (int)hc, (int)wc, map, hb, nbk, s);
+    else if (cur_dt == SS_F32) fe_gather<float>(cur, o.dtype, dst, (int)h, (int)w, c, r0, c0, (int)hc, (int)wc, map, hb, nbk, s);
+    else if (cur_dt == SS_U16) fe_gather<uint16_t>(cur, o.dtype, dst, (int)h, (int)w, c, r0, c0, (int)hc, (int)wc, map, hb, nbk, s);
+    else fe_gather<__half>(cur, o.dtype, dst, (int)h, (int)w, c, r0, c0, (int)hc, (int)wc, map, hb, nbk, s);
     SS_CK(cudaGetLastError());
   }
   SS_CK(cudaStreamSynchronize(s));

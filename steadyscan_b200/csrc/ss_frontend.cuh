@@ -203,7 +203,8 @@ __global__ void k_frame_divide(double* __restrict__ x, size_t per_frame, size_t 
 
 // Block matrices of frames: out (Hb x nb * n) entry (r, b + f nb) = frame f's cropped pixel
 // gather[r + b Hb] (column-major in the cropped hc x wc frame; -1: 0), the cropped frame being rows
-// [r0, r0 + hc) and columns [c0, c0 + wc) of the h x w frame.
+// [r0, r0 + hc) and columns [c0, c0 + wc) of the h x w frame. For maps without row structure
+// (k_block_rows); the reads follow the map, the writes are coalesced.
 template <class InT, class OutT>
 __global__ void __launch_bounds__(256) k_block_gather(const void* __restrict__ in, OutT* __restrict__ out, int h, int w,
                                                       int n, int r0, int c0, int hc, const int* __restrict__ gather,
@@ -221,6 +222,109 @@ __global__ void __launch_bounds__(256) k_block_gather(const void* __restrict__ i
     }
     out[e] = v;
   }
+}
+
+// Block matrices of a map whose blocks are runs of whole lines: block b holds the cropped rows
+// [start[b], start[b + 1]), entry r being row r mod k_b of column r div k_b (k_b = start[b+1] -
+// start[b]), zeros past column wc - 1. That is the reference's map of a scan with a whole number of
+// lines per knot, and a transpose in memory: the frame is column-major along the lines, a block along
+// the pixels. Bound: HBM, with instruction issue close behind for 16-bit samples. A CTA moves a tile
+// of bt consecutive blocks (at most kRowTile rows) by kRowTile columns through shared memory, so that
+// reads run down the columns (VE samples, 16 bytes, per thread where every tile's first row and column
+// is aligned) and writes along the blocks (VO entries, 16 bytes, per thread where hb is a multiple of
+// VO); reading the map's strided pixels directly used 4 of the 32 bytes of each sector. Tile column j
+// starts at word j * pitch + j / 4: the 4 columns of a thread's 8 entries (2 lines per block) then
+// fall into different banks across the warp. K > 0: every block has K lines and the index arithmetic
+// is shifts and constants (the default scan's 1, 2 and 4 lines per knot). Grid: (block tiles, column
+// tiles, frames).
+constexpr int kRowTile = 64;
+constexpr int kRowMaxLines = 32;  // longer runs are coalesced already in k_block_gather
+template <class InT, class OutT, int VE, int VO, int K>
+__global__ void __launch_bounds__(256) k_block_rows(const InT* __restrict__ in, OutT* __restrict__ out, int h, int w,
+                                                    int r0, int c0, int wc, const int* __restrict__ start, int hb,
+                                                    int nb, int bt, int slots, unsigned slots_inv) {
+  constexpr int kWord = sizeof(InT) < 4 ? 4 / sizeof(InT) : 1;  // samples of a tile word
+  constexpr int kPitch = kRowTile + kWord;                      // an odd number of words
+  __shared__ __align__(16) InT tile[kRowTile * kPitch + (kRowTile / 4) * kWord];
+  __shared__ int s_k[kRowTile], s_m[kRowTile], s_off[kRowTile];
+  auto col = [](int j) { return j * kPitch + (j >> 2) * kWord; };
+  const int b0 = blockIdx.x * bt, nbt = min(bt, nb - b0);
+  const int j0 = blockIdx.y * kRowTile, nc = min(kRowTile, wc - j0);
+  const size_t f = blockIdx.z;
+  const int row0 = start[b0], rows = start[b0 + nbt] - row0;
+  const InT* src = in + f * (size_t)h * w + (size_t)(j0 + c0) * h + (row0 + r0);
+  constexpr int kVecs = kRowTile / VE;  // vectors of a tile column
+#pragma unroll 4
+  for (int idx = threadIdx.x; idx < nc * kVecs; idx += 256) {
+    const int j = idx / kVecs, i = (idx % kVecs) * VE;
+    if (i >= rows) continue;
+    if constexpr (VE == 1) {
+      tile[col(j) + i] = src[(size_t)j * h + i];
+    } else if constexpr (sizeof(InT) == 8) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(src + (size_t)j * h + i));
+      const InT* e = reinterpret_cast<const InT*>(&v);
+#pragma unroll
+      for (int q = 0; q < VE; q++) tile[col(j) + i + q] = e[q];
+    } else {  // whole words
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(src + (size_t)j * h + i));
+      uint32_t* t = reinterpret_cast<uint32_t*>(tile + col(j) + i);
+      t[0] = v.x; t[1] = v.y; t[2] = v.z; t[3] = v.w;
+    }
+  }
+  if (K == 0 && (int)threadIdx.x < nbt) {
+    const int s = start[b0 + threadIdx.x], k = start[b0 + threadIdx.x + 1] - s;
+    s_k[threadIdx.x] = k;
+    s_m[threadIdx.x] = (65536 + k - 1) / k;  // e / k == (e * m) >> 16 for e < 64 * 32, k <= 32
+    s_off[threadIdx.x] = s - row0;
+  }
+  __syncthreads();
+  OutT* const fo = out + f * (size_t)hb * nb;
+  auto cvt = [](InT x) -> OutT {
+    if constexpr (std::is_same<InT, OutT>::value) return x;
+    else return (OutT)to_double(x);
+  };
+  // `slots` runs of VO entries per block, the thread's block idx / slots (by its rounded-up reciprocal)
+  const int ns = K ? kRowTile * K / VO : slots;
+#pragma unroll 2
+  for (int idx = threadIdx.x; idx < nbt * ns; idx += 256) {
+    const int bl = K ? idx / ns : (int)__umulhi((unsigned)idx, slots_inv), e0 = (idx - bl * ns) * VO;
+    const int k = K ? K : s_k[bl], off = K ? bl * K : s_off[bl], left = nc * k - e0;
+    if (left <= 0) continue;
+    const int m = K ? 0 : s_m[bl];
+    auto col_of = [&](int e) { return K ? e / k : (e * m) >> 16; };
+    struct alignas(VO * sizeof(OutT)) Run { OutT v[VO]; } run;
+    if (kWord == 2 && VO > 1 && ((k | off) & 1) == 0) {  // both lines of a pair of entries in one word
+#pragma unroll
+      for (int q = 0; q < VO; q += 2) {
+        const int e = e0 + q, j = col_of(e);  // past the columns: stale tile entries, not stored
+        const uint32_t wd = *reinterpret_cast<const uint32_t*>(tile + col(j) + off + (e - j * k));
+        if constexpr (std::is_same<InT, OutT>::value && VO > 1) {
+          reinterpret_cast<uint32_t*>(&run)[q / 2] = wd;
+        } else {
+          const InT* x = reinterpret_cast<const InT*>(&wd);
+          run.v[q] = cvt(x[0]);
+          run.v[q + 1 < VO ? q + 1 : q] = cvt(x[1]);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < VO; q++) {
+        const int e = e0 + q, j = col_of(e);
+        run.v[q] = cvt(tile[col(j) + off + (e - j * k)]);
+      }
+    }
+    OutT* o = fo + (size_t)(b0 + bl) * hb + (size_t)j0 * k + e0;
+    if (left >= VO) {
+      *reinterpret_cast<Run*>(o) = run;
+    } else {
+#pragma unroll
+      for (int q = 0; q < VO; q++)
+        if (q < left) o[q] = run.v[q];
+    }
+  }
+  if (j0 + kRowTile >= wc)  // the block's last column tile: zeros past its pixels
+    for (int bl = threadIdx.x >> 5; bl < nbt; bl += 8)
+      for (int r = (K ? K : s_k[bl]) * wc + (threadIdx.x & 31); r < hb; r += 32) fo[(size_t)(b0 + bl) * hb + r] = OutT(0);
 }
 
 }  // namespace ss
