@@ -2371,18 +2371,34 @@ static std::vector<double> blur_taps(double sd, int period, int* r_out) {
   return t;
 }
 
-template <class T>
-__global__ void k_to_f64(const void* __restrict__ in, double* __restrict__ out, size_t n) {
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
-    out[e] = to_double(reinterpret_cast<const T*>(in)[e]);
+// Both blur passes of n frames: src (InT) -> w1 -> w2; with stats, each frame's key range of w2.
+template <class InT>
+static cudaError_t fe_blur(const void* in, double* w1, double* w2, int h, int w, int n, int ph, int pw,
+                           const double* ty, int ry, const double* tx, int rx, unsigned* stats,
+                           cudaStream_t s) {
+  if (ry <= kBlurMaxR) {
+    const cudaError_t e = smem_attr(k_blur_cols<InT>, (int)blur_cols_smem(kBlurMaxR));
+    if (e != cudaSuccess) return e;
+    const dim3 grid((h + kBlurSeg - 1) / kBlurSeg, (w + 7) / 8, n);
+    k_blur_cols<InT><<<grid, 256, blur_cols_smem(ry), s>>>(static_cast<const InT*>(in), w1, h, w, ph, ty, ry);
+  } else {
+    k_blur_pass<InT, 0><<<dim3((h + 255) / 256, w, n), 256, 0, s>>>(in, w1, h, w, ph, ty, ry);
+  }
+  if (rx <= kBlurMaxR) {
+    const cudaError_t e = smem_attr(k_blur_rows, (int)blur_rows_smem(kBlurMaxR));
+    if (e != cudaSuccess) return e;
+    const dim3 grid((h + 31) / 32, (w + kBlurCols - 1) / kBlurCols, n);
+    k_blur_rows<<<grid, 256, blur_rows_smem(rx), s>>>(w1, w2, h, w, pw, tx, rx, stats);
+  } else {
+    k_blur_pass<double, 1><<<dim3((h + 255) / 256, w, n), 256, 0, s>>>(w1, w2, h, w, pw, tx, rx);
+    if (stats) k_frame_range<double><<<dim3(64, n), 256, 0, s>>>(w2, (size_t)h * w, stats);
+  }
+  return cudaGetLastError();
 }
 
-template <class InT>
-static void fe_blur(const void* in, double* w1, double* w2, int h, int w, int n, int ph, int pw, const double* ty,
-                    int ry, const double* tx, int rx, cudaStream_t s) {
-  const dim3 grid((h + 255) / 256, w, n);
-  k_blur_pass<InT, 0><<<grid, 256, 0, s>>>(in, w1, h, w, ph, ty, ry);
-  k_blur_pass<double, 1><<<grid, 256, 0, s>>>(w1, w2, h, w, pw, tx, rx);
+template <class T>
+static void fe_median(const void* x, size_t npx, int n, const unsigned* stats, double* med, cudaStream_t s) {
+  k_frame_median<T><<<kMedCtas * n, kMedThreads, 0, s>>>(static_cast<const T*>(x), npx, stats, med);
 }
 
 // Recognises a block map of whole lines (k_block_rows): fills start (nb + 1 cropped rows) and returns
@@ -2418,9 +2434,9 @@ struct BlockMap {
 
 template <class InT, class OutT>
 static void fe_gather_to(const InT* in, OutT* out, int h, int w, int n, int r0, int c0, int hc, int wc,
-                         const BlockMap& map, int hb, int nb, cudaStream_t s) {
+                         const BlockMap& map, int hb, int nb, const double* med, cudaStream_t s) {
   if (!map.kmax) {
-    k_block_gather<InT, OutT><<<148 * 8, 256, 0, s>>>(in, out, h, w, n, r0, c0, hc, map.d, hb, nb);
+    k_block_gather<InT, OutT><<<148 * 8, 256, 0, s>>>(in, out, h, w, n, r0, c0, hc, map.d, hb, nb, med);
     return;
   }
   constexpr int kVec = 16 / sizeof(InT);
@@ -2431,8 +2447,9 @@ static void fe_gather_to(const InT* in, OutT* out, int h, int w, int n, int r0, 
   const dim3 grid((nb + map.bt - 1) / map.bt, (wc + kRowTile - 1) / kRowTile, n);
   const int slots = kRowTile * map.kmax / (wide ? kOut : 1);
   const unsigned inv = (unsigned)((0x100000000ull + slots - 1) / slots);
-#define SS_ROWS(VE, VO, K) \
-  k_block_rows<InT, OutT, VE, VO, K><<<grid, 256, 0, s>>>(in, out, h, w, r0, c0, wc, map.d, hb, nb, map.bt, slots, inv)
+#define SS_ROWS(VE, VO, K)                                                                                         \
+  k_block_rows<InT, OutT, VE, VO, K>                                                                             \
+      <<<grid, 256, 0, s>>>(in, out, h, w, r0, c0, wc, map.d, hb, nb, map.bt, slots, inv, med)
   const int k = (map.start[nb] - map.start[0]) == nb * map.kmax ? map.kmax : 0;  // every block has k lines
   if (vec && wide && k == 1) SS_ROWS(kVec, kOut, 1);
   else if (vec && wide && k == 2) SS_ROWS(kVec, kOut, 2);
@@ -2446,11 +2463,11 @@ static void fe_gather_to(const InT* in, OutT* out, int h, int w, int n, int r0, 
 
 template <class InT>
 static void fe_gather(const void* in, int out_dt, void* out, int h, int w, int n, int r0, int c0, int hc, int wc,
-                      const BlockMap& map, int hb, int nb, cudaStream_t s) {
+                      const BlockMap& map, int hb, int nb, const double* med, cudaStream_t s) {
   const InT* x = static_cast<const InT*>(in);
-  if (out_dt == SS_F64) fe_gather_to(x, (double*)out, h, w, n, r0, c0, hc, wc, map, hb, nb, s);
-  else if (out_dt == SS_F32) fe_gather_to(x, (float*)out, h, w, n, r0, c0, hc, wc, map, hb, nb, s);
-  else fe_gather_to(x, (uint16_t*)out, h, w, n, r0, c0, hc, wc, map, hb, nb, s);
+  if (out_dt == SS_F64) fe_gather_to(x, (double*)out, h, w, n, r0, c0, hc, wc, map, hb, nb, med, s);
+  else if (out_dt == SS_F32) fe_gather_to(x, (float*)out, h, w, n, r0, c0, hc, wc, map, hb, nb, med, s);
+  else fe_gather_to(x, (uint16_t*)out, h, w, n, r0, c0, hc, wc, map, hb, nb, med, s);
 }
 
 int prepare_frames(const ss_prep_frames* p) {
@@ -2511,8 +2528,13 @@ int prepare_frames(const ss_prep_frames* p) {
     tx = blur_taps(sd, pw, &rx);
   }
   const size_t fsz = dtype_size(fdt), osz = dtype_size(o.dtype), npx = (size_t)h * w;
-  // frames per pass: about 1 GB of FP64 work memory, and the blur grid's z extent
-  const int chunk = (int)std::max<size_t>(1, std::min<size_t>({(size_t)n, ((size_t)1 << 30) / (16 * npx), (size_t)65535}));
+  // Frames per pass: about 1 GB for the two FP64 planes of the blur (passes small enough for their
+  // planes to stay in L2 were slower: 256 frames of 512 x 512 in parts of 64 MB 2420 us, in one 1740 us),
+  // a host upload bounded by 128 MB, and the frame is the grid's z extent.
+  size_t per_pass = 65535;
+  if (blur) per_pass = std::min(per_pass, ((size_t)1 << 30) / (16 * npx));
+  if (p->frames.location == SS_HOST) per_pass = std::min(per_pass, ((size_t)128 << 20) / (fsz * npx));
+  const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)n, per_pass));
   CallMem m;
   SS_CK(cudaStreamCreateWithFlags(&m.s, cudaStreamNonBlocking));
   cudaStream_t s = m.s;
@@ -2520,11 +2542,12 @@ int prepare_frames(const ss_prep_frames* p) {
   int* d_gather = m.take<int>(map_n);
   double* d_taps = blur ? m.take<double>(ty.size() + tx.size()) : nullptr;
   void* d_raw = p->frames.location == SS_HOST ? m.take<char>(fsz * npx * chunk) : nullptr;
-  double* w1 = (blur || med) ? m.take<double>(npx * chunk) : nullptr;
+  double* w1 = blur ? m.take<double>(npx * chunk) : nullptr;
   double* w2 = blur ? m.take<double>(npx * chunk) : nullptr;
   double* d_med = med ? m.take<double>(chunk) : nullptr;
-  if (!d_gather || (blur && !d_taps) || (p->frames.location == SS_HOST && !d_raw) || ((blur || med) && !w1) ||
-      (blur && !w2) || (med && !d_med))
+  unsigned* d_stats = med ? m.take<unsigned>((size_t)kFrameStats * chunk) : nullptr;
+  if (!d_gather || (blur && !d_taps) || (p->frames.location == SS_HOST && !d_raw) || (blur && (!w1 || !w2)) ||
+      (med && (!d_med || !d_stats)))
     return fail(SS_ERR_OUT_OF_MEMORY, "prepare_frames: work memory");
   SS_CK(cudaMemcpyAsync(d_gather, map.kmax ? map.start.data() : p->gather, map_n * sizeof(int), cudaMemcpyHostToDevice,
                         s));
@@ -2542,7 +2565,6 @@ int prepare_frames(const ss_prep_frames* p) {
     SS_CK(cudaMemcpyAsync(d_taps + ty.size(), tx.data(), tx.size() * 8, cudaMemcpyHostToDevice, s));
   }
   const int r0 = cr[2], c0 = cr[0];
-  const int g = 148 * 8;
   for (int f0 = 0; f0 < n; f0 += chunk) {
     const int c = std::min(chunk, n - f0);
     const char* src = static_cast<const char*>(p->frames.data) + fsz * npx * f0;
@@ -2552,33 +2574,35 @@ int prepare_frames(const ss_prep_frames* p) {
     }
     const void* cur = src;
     int cur_dt = fdt;
+    if (med) SS_CK(cudaMemsetAsync(d_stats, 0xFF, (size_t)kFrameStats * c * 4, s));
     if (blur) {  // prefilter_foralignment's blur, then its samples in FP64
       const double* dty = d_taps;
       const double* dtx = d_taps + ty.size();
-      if (fdt == SS_F64) fe_blur<double>(src, w1, w2, (int)h, (int)w, c, ph, pw, dty, ry, dtx, rx, s);
-      else if (fdt == SS_F32) fe_blur<float>(src, w1, w2, (int)h, (int)w, c, ph, pw, dty, ry, dtx, rx, s);
-      else if (fdt == SS_U16) fe_blur<uint16_t>(src, w1, w2, (int)h, (int)w, c, ph, pw, dty, ry, dtx, rx, s);
-      else fe_blur<__half>(src, w1, w2, (int)h, (int)w, c, ph, pw, dty, ry, dtx, rx, s);
+      const int ih = (int)h, iw = (int)w;
+      if (fdt == SS_F64) SS_CK(fe_blur<double>(src, w1, w2, ih, iw, c, ph, pw, dty, ry, dtx, rx, d_stats, s));
+      else if (fdt == SS_F32) SS_CK(fe_blur<float>(src, w1, w2, ih, iw, c, ph, pw, dty, ry, dtx, rx, d_stats, s));
+      else if (fdt == SS_U16) SS_CK(fe_blur<uint16_t>(src, w1, w2, ih, iw, c, ph, pw, dty, ry, dtx, rx, d_stats, s));
+      else SS_CK(fe_blur<__half>(src, w1, w2, ih, iw, c, ph, pw, dty, ry, dtx, rx, d_stats, s));
       cur = w2;
       cur_dt = SS_F64;
-    } else if (med) {  // the median division works on FP64 samples
-      if (fdt == SS_F64) k_to_f64<double><<<g, 256, 0, s>>>(src, w1, npx * c);
-      else if (fdt == SS_F32) k_to_f64<float><<<g, 256, 0, s>>>(src, w1, npx * c);
-      else if (fdt == SS_U16) k_to_f64<uint16_t><<<g, 256, 0, s>>>(src, w1, npx * c);
-      else k_to_f64<__half><<<g, 256, 0, s>>>(src, w1, npx * c);
-      cur = w1;
-      cur_dt = SS_F64;
+    } else if (med) {
+      const dim3 rg((unsigned)std::min<size_t>(64, (npx + 255) / 256), c);
+      if (fdt == SS_F64) k_frame_range<double><<<rg, 256, 0, s>>>(static_cast<const double*>(cur), npx, d_stats);
+      else if (fdt == SS_F32) k_frame_range<float><<<rg, 256, 0, s>>>(static_cast<const float*>(cur), npx, d_stats);
+      else if (fdt == SS_U16) k_frame_range<uint16_t><<<rg, 256, 0, s>>>(static_cast<const uint16_t*>(cur), npx, d_stats);
+      else k_frame_range<__half><<<rg, 256, 0, s>>>(static_cast<const __half*>(cur), npx, d_stats);
     }
     if (med) {
-      double* x = const_cast<double*>(static_cast<const double*>(cur));
-      k_frame_median<double><<<c, 1024, 0, s>>>(x, npx, d_med);
-      k_frame_divide<<<g, 256, 0, s>>>(x, npx, npx * c, d_med);
+      if (cur_dt == SS_F64) fe_median<double>(cur, npx, c, d_stats, d_med, s);
+      else if (cur_dt == SS_F32) fe_median<float>(cur, npx, c, d_stats, d_med, s);
+      else if (cur_dt == SS_U16) fe_median<uint16_t>(cur, npx, c, d_stats, d_med, s);
+      else fe_median<__half>(cur, npx, c, d_stats, d_med, s);
     }
     void* dst = static_cast<char*>(const_cast<void*>(o.data)) + osz * (size_t)hb * nbk * f0;
-    if (cur_dt == SS_F64) fe_gather<double>(cur, o.dtype, dst, (int)h, (int)w, c, r0, c0, (int)hc, (int)wc, map, hb, nbk, s);
-    else if (cur_dt == SS_F32) fe_gather<float>(cur, o.dtype, dst, (int)h, (int)w, c, r0, c0, (int)hc, (int)wc, map, hb, nbk, s);
-    else if (cur_dt == SS_U16) fe_gather<uint16_t>(cur, o.dtype, dst, (int)h, (int)w, c, r0, c0, (int)hc, (int)wc, map, hb, nbk, s);
-    else fe_gather<__half>(cur, o.dtype, dst, (int)h, (int)w, c, r0, c0, (int)hc, (int)wc, map, hb, nbk, s);
+    if (cur_dt == SS_F64) fe_gather<double>(cur, o.dtype, dst, (int)h, (int)w, c, r0, c0, (int)hc, (int)wc, map, hb, nbk, d_med, s);
+    else if (cur_dt == SS_F32) fe_gather<float>(cur, o.dtype, dst, (int)h, (int)w, c, r0, c0, (int)hc, (int)wc, map, hb, nbk, d_med, s);
+    else if (cur_dt == SS_U16) fe_gather<uint16_t>(cur, o.dtype, dst, (int)h, (int)w, c, r0, c0, (int)hc, (int)wc, map, hb, nbk, d_med, s);
+    else fe_gather<__half>(cur, o.dtype, dst, (int)h, (int)w, c, r0, c0, (int)hc, (int)wc, map, hb, nbk, d_med, s);
     SS_CK(cudaGetLastError());
   }
   SS_CK(cudaStreamSynchronize(s));

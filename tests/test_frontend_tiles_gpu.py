@@ -55,3 +55,63 @@ def test_a_map_that_only_starts_like_whole_lines_is_gathered():
     lay.prevknotind = blk
     got = api.prepare_frames(_device(frames), lay, out_dtype=np.float32).cpu().numpy()
     np.testing.assert_array_equal(got, frontend.set_bmdata(frames, blk, nb, [0, 0, 0, 0], 0.0, False).astype(np.float32))
+
+
+# a warp's 256 outputs down a column and a CTA's 64 columns full, one short and one over; windows that
+# wrap more than once round a small frame; a window too wide for the tiles (R > 320)
+BLURS = [(256, 64, 1.0), (257, 65, 2.0), (255, 63, 0.3), (7, 5, 1.5), (33, 129, 6.0), (720, 40, 36.0), (513, 9, 4.7)]
+
+
+@pytest.mark.parametrize("h,w,sd", BLURS)
+@pytest.mark.parametrize("src", [np.uint16, np.float32])
+def test_blur_tiles_match_the_fft(h, w, sd, src):
+    """The FFT and the direct sums round differently, each by a few 1e-16 of the largest sample."""
+    frames = _frames(h, w, 2, src, seed=h)
+    lay = _rows_layout(h, w, h, [0, 0, 0, 0])
+    got = api.prepare_frames(_device(frames), lay, pregauss=sd).cpu().numpy()
+    ref = frontend.set_bmdata(frames, lay.prevknotind, h, lay.cropping, sd, False)
+    np.testing.assert_allclose(got, ref, rtol=1e-12, atol=1e-12 * np.abs(ref).max())
+
+
+def _median_frames(kind, h, w):
+    rng = np.random.default_rng(h * 7 + w)
+    x = rng.uniform(10, 200, size=(h, w, 2))
+    if kind == "ties":  # a few values, many samples each: no range of keys narrows to a few samples
+        x = np.floor(x / 50) * 50 + 1
+    elif kind == "halves":  # the two middle samples on either side of a gap
+        x = np.where((np.arange(h * w) % 2 == 0).reshape(h, w)[:, :, None], 3.0, 1e9) * np.ones(2)
+    elif kind == "constant":
+        x = np.full_like(x, 4.25)
+    elif kind == "wide":  # both signs, every binade, zeros of both signs and infinities
+        x = np.ldexp(rng.standard_normal(x.shape), rng.integers(-900, 900, x.shape))
+        x.reshape(-1)[::7] = 0.0
+        x.reshape(-1)[3::11] = -0.0
+        x[0, 0], x[-1, -1] = np.inf, -np.inf
+        x += 1.5  # the median of symmetric samples would be next to zero
+    elif kind == "nan":
+        x[h // 2, w // 2, 1] = np.nan
+    return x
+
+
+# counts at and around the 1024 samples that are ranked at once, odd and even, one sample
+@pytest.mark.parametrize("h,w", [(1, 1), (1, 2), (32, 32), (41, 25), (31, 33), (300, 217), (128, 512)])
+@pytest.mark.parametrize("kind", ["plain", "ties", "halves", "constant", "wide", "nan"])
+def test_median_is_exact(kind, h, w):
+    frames = _median_frames(kind, h, w)
+    lay = _rows_layout(h, w, h, [0, 0, 0, 0])
+    got = api.prepare_frames(_device(frames), lay, mednorm=True).cpu().numpy()
+    with np.errstate(all="ignore"):
+        med = np.median(frames.reshape(h * w, 2, order="F"), axis=0)
+        ref = frames / med
+    np.testing.assert_array_equal(got, frontend.set_bmdata(ref, lay.prevknotind, h, lay.cropping, 0.0, False))
+
+
+@pytest.mark.parametrize("src", [np.uint16, np.float32, np.float16])
+def test_median_of_storage_types(src):
+    frames = (np.random.default_rng(5).integers(1, 900, size=(90, 61, 3))).astype(src)
+    lay = _rows_layout(90, 61, 30, [0, 0, 0, 0])
+    got = api.prepare_frames(_device(frames), lay, mednorm=True, out_dtype=np.float32).cpu().numpy()
+    f = frames.astype(np.float64)
+    ref = frontend.set_bmdata(f / np.median(f.reshape(-1, 3, order="F"), axis=0), lay.prevknotind, 30, lay.cropping,
+                              0.0, False)
+    np.testing.assert_array_equal(got, ref.astype(np.float32))
