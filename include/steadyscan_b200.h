@@ -239,7 +239,8 @@ SS_API void ss_server_destroy(ss_server* server);
  * device. All pointers are device memory of the current device: diag n x 3 (xx, yy, xy), coupling
  * (n-1) x 4 ([[c0 c2] [c3 c1]] between block i and block i+1), rhs and x n x 2, row-major.
  * stream is a cudaStream_t (NULL: the legacy default stream); the call returns after the solve.
- * The workspace (104 bytes per block) is allocated and freed inside the call. */
+ * The workspace (104 bytes per block) comes from the library's memory pool of the device and goes
+ * back to it inside the call; the pool keeps it for the next call. */
 SS_API int ss_solve_block_tridiagonal(int32_t n, const double* diag, const double* coupling, const double* rhs,
                                       double* x, void* stream);
 
@@ -251,8 +252,7 @@ SS_API int ss_solve_block_tridiagonal(int32_t n, const double* diag, const doubl
  * ss_solve_block_tridiagonal; the workspace is a fixed device array inside this library of
  * 32768 blocks (3.4 MB, held by every GPU that loads the library until the process exits), so
  * n > 32768 is rejected with SS_ERR_INVALID_ARGUMENT. The first call on a device looks up that
- * array's device address and sets the solve kernel's shared-memory attribute (again after the
- * device's context has been reset, e.g. by cudaDeviceReset). Each call waits for `stream`
+ * array's device address (again after the device's context has been reset, e.g. by cudaDeviceReset). Each call waits for `stream`
  * (cudaStreamSynchronize) before it returns. All calls
  * share the one array per device: calls that overlap on the GPU (different streams or threads at
  * the same time) race and corrupt each other's results; serialize them. Each call writes every part

@@ -1416,9 +1416,11 @@ static int reset_state(Batch::Impl* b) {
   return SS_OK;
 }
 
-// Dynamic shared memory of k_solve_system and k_block_tridiag: the separator system of the partitioned
-// solve and the partitions' first-interior relations.
-constexpr size_t kSolveSmem = (size_t)kSolveThreads * kPartSmemStride * sizeof(double);
+// Dynamic shared memory of a CTA of k_solve_system and of k_block_tridiag: its part of the separator
+// system of the partitioned solve and its partitions' first-interior relations.
+constexpr size_t kSolveSmem = (size_t)kSolveSysThreads * kPartSmemStride * sizeof(double);
+constexpr size_t kTridiagSmem = (size_t)kTridiagThreads * kPartSmemStride * sizeof(double);
+static_assert(kTridiagSmem <= 48 * 1024, "no opt-in");
 
 // The half-step solve of every group in phase kPhHalf: set-up over kSolveSplit CTAs per group,
 // compaction in one CTA, the blocks over kSolveSplit CTAs, the partitioned solve and filters in one
@@ -1428,12 +1430,9 @@ static void solve_launch(cudaStream_t s, const GroupDesc* gd, GroupCtl* ctl, int
   k_solve_prep<<<split, kSolvePrepThreads, 0, s>>>(gd, ctl);
   k_solve_compact<<<nG, kSolveThreads, 0, s>>>(gd, ctl);
   k_solve_planes<<<split, kSolvePrepThreads, 0, s>>>(gd, ctl);
-  k_solve_system<<<nG, kSolveThreads, kSolveSmem, s>>>(gd, ctl);
+  k_solve_system<<<nG * kSolveCluster, kSolveSysThreads, kSolveSmem, s>>>(gd, ctl);
   k_solve_expand<<<split, kSolvePrepThreads, 0, s>>>(gd, ctl);
 }
-
-// Opts k_block_tridiag into kSolveSmem of dynamic shared memory.
-static cudaError_t block_tridiag_attr() { return smem_attr(k_block_tridiag, (int)kSolveSmem); }
 
 // Trial rounds per cycle of the precision 'S' line search: the first cycle's, and the range of the
 // later ones (set from the longest search that ended in the cycle before).
@@ -1484,7 +1483,7 @@ static int enqueue_cycle(Batch::Impl* b) {
     b->fmark(5);
     k_solve_planes<<<split, kSolvePrepThreads, 0, s>>>(b->d_gd, b->d_ctl);
     b->fmark(7);
-    k_solve_system<<<nG, kSolveThreads, kSolveSmem, s>>>(b->d_gd, b->d_ctl);
+    k_solve_system<<<nG * kSolveCluster, kSolveSysThreads, kSolveSmem, s>>>(b->d_gd, b->d_ctl);
     b->fmark(8);
     k_solve_expand<<<split, kSolvePrepThreads, 0, s>>>(b->d_gd, b->d_ctl);
   } else {
@@ -1597,7 +1596,6 @@ static int capture_while(cudaStream_t s, cudaGraphConditionalHandle h, cudaGraph
 
 // Opts every kernel of the run into its shared memory before capture (no attribute calls inside).
 static int prime_attributes(Batch::Impl* b) {
-  SS_CK(smem_attr(k_solve_system, (int)kSolveSmem));
   SS_CK(b->ks.eval(kAssemble, 0, b->stream, b->d_gd, b->d_sched, b->n_chunks, b->d_ctl, b->max_hb, b->win_bytes));
   if (b->ks.round)
     SS_CK(b->ks.round(0, b->stream, b->d_gd, b->d_tsched, b->n_frames_total, (int)b->gd.size(), b->d_ctl,
@@ -1696,7 +1694,6 @@ int Batch::start() {
   b->t_start = std::chrono::steady_clock::now();
   SS_CK(cudaSetDevice(b->device));
   if (!b->h_counters) SS_CK(cudaHostAlloc(&b->h_counters, (kCounters + 1) * sizeof(int), cudaHostAllocDefault));
-  SS_CK(smem_attr(k_solve_system, (int)kSolveSmem));
   int rc = reset_state(b);
   if (rc) return rc;
   b->cycles = 0;
@@ -2123,7 +2120,6 @@ int Server::step() {
   if (v->n_tiles == 0) return SS_OK;  // nothing to run
   cudaStream_t s = v->stream;
   const int nG = v->capacity;
-  SS_CK(smem_attr(k_solve_system, (int)kSolveSmem));
   v->cycles++;
   int* sc = v->d_sched;
   const int nc = v->n_chunks;
@@ -3102,9 +3098,7 @@ int ss_solve_block_tridiagonal_noalloc(int32_t n, const double* diag, const doub
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // every node of the workspace that the solve reads is written first by k_block_tridiag
-  cudaError_t ea = ss::block_tridiag_attr();
-  if (ea != cudaSuccess) return ss::fail(SS_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea));
-  ss::k_block_tridiag<<<1, ss::kSolveThreads, ss::kSolveSmem, s>>>(n, diag, coupling, rhs, x, work);
+  ss::k_block_tridiag<<<ss::kSolveCluster, ss::kTridiagThreads, ss::kTridiagSmem, s>>>(n, diag, coupling, rhs, x, work);
   cudaError_t e = cudaGetLastError();
   cudaError_t e2 = cudaStreamSynchronize(s);
   if (e != cudaSuccess || e2 != cudaSuccess)
@@ -3120,11 +3114,16 @@ int ss_solve_block_tridiagonal(int32_t n, const double* diag, const double* coup
     return ss::fail(SS_ERR_INVALID_ARGUMENT, "ss_solve_block_tridiagonal: bad arguments");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   double* work = nullptr;
-  cudaError_t e = cudaMallocAsync(&work, (size_t)n * ss::kCrStride * sizeof(double), s);
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return ss::fail(SS_ERR_CUDA, std::string("cudaGetDevice: ") + cudaGetErrorString(e));
+  // from the library's pool, which keeps it for the next call (the default pool gives its memory back
+  // to the device at every synchronisation: 400 us of a call)
+  cudaMemPool_t pool = ss::work_pool(dev);
+  if (!pool) return ss::fail(SS_ERR_OUT_OF_MEMORY, "workspace: no device memory pool");
+  e = cudaMallocFromPoolAsync((void**)&work, (size_t)n * ss::kCrStride * sizeof(double), pool, s);
   if (e != cudaSuccess) return ss::fail(SS_ERR_OUT_OF_MEMORY, std::string("workspace: ") + cudaGetErrorString(e));
-  cudaError_t ea = ss::block_tridiag_attr();
-  if (ea != cudaSuccess) return ss::fail(SS_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea));
-  ss::k_block_tridiag<<<1, ss::kSolveThreads, ss::kSolveSmem, s>>>(n, diag, coupling, rhs, x, work);
+  ss::k_block_tridiag<<<ss::kSolveCluster, ss::kTridiagThreads, ss::kTridiagSmem, s>>>(n, diag, coupling, rhs, x, work);
   e = cudaGetLastError();
   cudaError_t e2 = cudaFreeAsync(work, s);
   cudaError_t e3 = cudaStreamSynchronize(s);

@@ -9,6 +9,13 @@ namespace ss {
 constexpr int kSolveThreads = 1024;
 constexpr int kCrStride = 13;  // D(3: xx yy xy) L(4) R(4) b(2)
 
+// The CTAs of a solve cluster: a chain is solved by up to kSolveCluster CTAs that hold its separator
+// system in their shared memory together. One 1024-thread CTA per chain was bound by that SM's memory
+// queue (16385 knots: 158 us per half-step solve; ss_solve_block_tridiagonal of 16385 blocks 670 us
+// with its allocation, now 68 us).
+constexpr int kSolveCluster = 8;
+constexpr int kSolveSysThreads = kSolveThreads / kSolveCluster;  // a partition per thread of the cluster
+
 __device__ __forceinline__ void cr_load(const double* n, double& d0, double& d1, double& d2, M2& L, M2& R, double& b0,
                                         double& b1) {
   d0 = n[0]; d1 = n[1]; d2 = n[2];
@@ -18,28 +25,33 @@ __device__ __forceinline__ void cr_load(const double* n, double& d0, double& d1,
 }
 
 // Solves a symmetric positive definite block-tridiagonal system with 2x2 blocks in place by block
-// cyclic reduction, with the whole CTA. Node i of cr holds (D_i: xx yy xy, L_i: coupling to its left
+// cyclic reduction, with the first `ranks` CTAs of a cluster (all their threads call). Node i is held by
+// thread i of the cluster in its CTA's part of cr: (D_i: xx yy xy, L_i: coupling to its left
 // neighbour, R_i: coupling to its right neighbour, b_i) in kCrStride doubles; on return b_i holds
 // x_i. At stride s every multiple of 2s absorbs its two odd-multiple neighbours (each elimination is
 // a Schur complement on 2x2 blocks), so the reduction takes ceil(log2 h) levels; back substitution
 // runs the levels in reverse. In exact arithmetic this is the LDL^T of the system in a nested
 // dissection order, so it solves the same equations as the reference's exact sparse solvers
 // (eigensolve.cpp:35-38, cusolversolver.cu:53-56).
-__device__ void cr_solve(double* cr, int h) {
-  const int t = threadIdx.x, nt = blockDim.x;
+__device__ void cr_solve(cg::cluster_group& cluster, double* cr, int h) {
+  const int bd = blockDim.x, i = (int)cluster.block_rank() * bd + threadIdx.x;
+  auto node = [&](int j) -> double* {
+    const int q = j / bd;
+    return cluster.map_shared_rank(cr, q) + (size_t)(j - q * bd) * kCrStride;
+  };
   int top = 1;
   while (top < h) top <<= 1;
+  double* const n = cr + (size_t)threadIdx.x * kCrStride;
   for (int s = 1; s < h; s <<= 1) {
-    for (int j = t * 2 * s; j < h; j += nt * 2 * s) {
-      double* n = cr + (size_t)j * kCrStride;
+    if (i < h && (i & (2 * s - 1)) == 0) {
       double d0, d1, d2, b0, b1;
       M2 L, R;
       cr_load(n, d0, d1, d2, L, R, b0, b1);
       M2 D = {d0, d2, d2, d1};
-      if (j - s >= 0) {
+      if (i - s >= 0) {
         double e0, e1, e2, c0, c1;
         M2 Ll, Rl;
-        cr_load(cr + (size_t)(j - s) * kCrStride, e0, e1, e2, Ll, Rl, c0, c1);
+        cr_load(node(i - s), e0, e1, e2, Ll, Rl, c0, c1);
         M2 Di = m2_inv({e0, e2, e2, e1});
         M2 T = m2_mul(L, Di);
         D = m2_sub(D, m2_mul(T, Rl));
@@ -47,10 +59,10 @@ __device__ void cr_solve(double* cr, int h) {
         b1 -= T.c * c0 + T.d * c1;
         L = m2_neg(m2_mul(T, Ll));
       }
-      if (j + s < h) {
+      if (i + s < h) {
         double e0, e1, e2, c0, c1;
         M2 Lr, Rr;
-        cr_load(cr + (size_t)(j + s) * kCrStride, e0, e1, e2, Lr, Rr, c0, c1);
+        cr_load(node(i + s), e0, e1, e2, Lr, Rr, c0, c1);
         M2 Di = m2_inv({e0, e2, e2, e1});
         M2 T = m2_mul(R, Di);
         D = m2_sub(D, m2_mul(T, Lr));
@@ -63,27 +75,25 @@ __device__ void cr_solve(double* cr, int h) {
       n[7] = R.a; n[8] = R.b; n[9] = R.c; n[10] = R.d;
       n[11] = b0; n[12] = b1;
     }
-    __syncthreads();
+    cluster.sync();
   }
-  if (t == 0 && h > 0) {
-    double* n = cr;
+  if (i == 0 && h > 0) {
     M2 Di = m2_inv({n[0], n[2], n[2], n[1]});
     double b0 = n[11], b1 = n[12];
     n[11] = Di.a * b0 + Di.b * b1;
     n[12] = Di.c * b0 + Di.d * b1;
   }
-  __syncthreads();
+  cluster.sync();
   for (int s = top >> 1; s >= 1; s >>= 1) {
-    for (int i = s + t * 2 * s; i < h; i += nt * 2 * s) {
-      double* n = cr + (size_t)i * kCrStride;
+    if (i < h && (i & (2 * s - 1)) == s) {
       double d0, d1, d2, b0, b1;
       M2 L, R;
       cr_load(n, d0, d1, d2, L, R, b0, b1);
-      const double* l = cr + (size_t)(i - s) * kCrStride;
+      const double* l = node(i - s);
       b0 -= L.a * l[11] + L.b * l[12];
       b1 -= L.c * l[11] + L.d * l[12];
       if (i + s < h) {
-        const double* r = cr + (size_t)(i + s) * kCrStride;
+        const double* r = node(i + s);
         b0 -= R.a * r[11] + R.b * r[12];
         b1 -= R.c * r[11] + R.d * r[12];
       }
@@ -91,10 +101,9 @@ __device__ void cr_solve(double* cr, int h) {
       n[11] = Di.a * b0 + Di.b * b1;
       n[12] = Di.c * b0 + Di.d * b1;
     }
-    __syncthreads();
+    cluster.sync();
   }
 }
-
 
 __device__ __forceinline__ M2 m2_t(const M2& x) { return {x.a, x.c, x.b, x.d}; }
 __device__ __forceinline__ M2 m2_add(const M2& x, const M2& y) { return {x.a + y.a, x.b + y.b, x.c + y.c, x.d + y.d}; }
@@ -105,7 +114,7 @@ __device__ __forceinline__ void m2_mv(const M2& m, double v0, double v1, double&
 __device__ __forceinline__ M2 sym_inv(double d0, double d1, double d2) { return m2_inv({d0, d2, d2, d1}); }
 
 // Node layout of the partitioned block-tridiagonal solve: the h nodes are split into P =
-// min(blockDim.x, h) contiguous partitions, the first rem = h - q P of q + 1 nodes and the rest of q;
+// min(threads of the cluster, h) contiguous partitions, the first rem = h - q P of q + 1 nodes and the rest of q;
 // every field of every node has a plane of h doubles in which node k of partition t sits at
 // k P + t, so the threads of a warp, each walking its own partition, touch consecutive doubles.
 constexpr int kRelStride = 10;                      // uL (4), uR (4), u0 (2)
@@ -136,21 +145,30 @@ struct PartLayout {
   }
 };
 
+// CTAs of a solve cluster that hold partitions of h nodes; the others leave at once (a cluster barrier
+// waits for the threads that have not exited), so a short chain pays for one CTA's barriers only.
+__device__ __forceinline__ int solve_ranks(int h) {
+  return min(kSolveCluster, max(1, (h + (int)blockDim.x - 1) / (int)blockDim.x));
+}
+
 // Solves the symmetric positive definite block-tridiagonal system of h nodes given in the planes
-// of pl (PartLayout of h and blockDim.x; L_i = R_{i-1}^T) with the whole CTA and writes x_i to
-// xo[i * xs] and yo[i * ys]. Partition method: thread t eliminates the interior of its partition
-// by block Thomas sweeps (backward for the relation of the first interior node, forward storing
-// D~^-1, S~ and b~), leaving its last node as separator; the separators' Schur complement is block
-// tridiagonal again and is solved by block cyclic reduction in shared memory (red: blockDim.x x
-// kCrStride doubles); the interior follows by back substitution. For SPD systems every block
-// elimination is a Schur complement of an SPD matrix, so this solves the same equations as the
-// reference's exact solvers (eigensolve.cpp:35-38, cusolversolver.cu:53-56) in another
-// elimination order. red holds blockDim.x x kPartSmemStride doubles: the separator system and
-// each partition's first-interior relation.
-__device__ void part_solve(double* pl, int h, double* red, double* xo, int xs, double* yo, int ys) {
-  const int t = threadIdx.x;
+// of pl (PartLayout of h and the cluster's threads; L_i = R_{i-1}^T) with the first solve_ranks(h) CTAs
+// of a cluster and writes x_i to xo[i * xs] and yo[i * ys]. Partition method: thread t eliminates the
+// interior of its partition by block Thomas sweeps (backward for the relation of the first interior
+// node, forward storing D~^-1, S~ and b~), leaving its last node as separator; the separators' Schur
+// complement is block tridiagonal again and is solved by block cyclic reduction in the CTAs' shared
+// memory; the interior follows by back substitution. For SPD systems every block elimination is a Schur
+// complement of an SPD matrix, so this solves the same equations as the reference's exact solvers
+// (eigensolve.cpp:35-38, cusolversolver.cu:53-56) in another elimination order. red holds blockDim.x x
+// kPartSmemStride doubles: this CTA's separators and its partitions' first-interior relations.
+// Bound by the serial chain of 2x2 inverses along a partition (a divide each); every sweep loads its
+// next node while it works on the current one.
+__device__ void part_solve(cg::cluster_group& cluster, double* pl, int h, double* red, double* xo, int xs, double* yo,
+                           int ys) {
   if (h <= 0) return;
-  const PartLayout L(h, blockDim.x);
+  const int bd = blockDim.x, tid = threadIdx.x;
+  const int t = (int)cluster.block_rank() * bd + tid;
+  const PartLayout L(h, bd * kSolveCluster);
   const int P = L.P;
   const bool own = t < P;
   const int mt = own ? L.m(t) : 0;
@@ -170,32 +188,43 @@ __device__ void part_solve(double* pl, int h, double* red, double* xo, int xs, d
   double* const S2 = pl + (size_t)kPS2 * h;
   double* const S3 = pl + (size_t)kPS3 * h;
   auto ldR = [&](size_t q) -> M2 { return {R0[q], R1[q], R2[q], R3[q]}; };
+  struct Node {
+    double d0, d1, d2, b0, b1;
+    M2 R;
+  };
+  auto ldN = [&](int k) -> Node {
+    const size_t q = L.pos(t, k);
+    return {D0[q], D1[q], D2[q], B0[q], B1[q], ldR(q)};
+  };
   const M2 Z = {0, 0, 0, 0};
   // coupling of node a to the previous separator (the last node of partition t - 1)
   const M2 La = (own && t > 0) ? m2_t(ldR(L.pos(t - 1, L.m(t - 1) - 1))) : Z;
+  double* const rel = red + (size_t)bd * kCrStride;
 
   // backward sweep: relation x_a = u0 + uL x_(previous separator) + uR x_e of the first interior node
   if (own && mt >= 2) {
-    size_t q = L.pos(t, mt - 2);
-    M2 Dc = {D0[q], D2[q], D2[q], D1[q]};
-    double b0 = B0[q], b1 = B1[q];
-    M2 S = ldR(q);
+    Node n = ldN(mt - 2);
+    M2 Dc = {n.d0, n.d2, n.d2, n.d1};
+    double b0 = n.b0, b1 = n.b1;
+    M2 S = n.R;
+    if (mt >= 3) n = ldN(mt - 3);
     for (int k = mt - 3; k >= 0; k--) {
-      q = L.pos(t, k);
-      const M2 Ri = ldR(q);
+      const Node nx = k > 0 ? ldN(k - 1) : n;
+      const M2 Ri = n.R;
       const M2 Nm = m2_mul(Ri, m2_inv(Dc));
-      Dc = m2_sub({D0[q], D2[q], D2[q], D1[q]}, m2_mul(Nm, m2_t(Ri)));
+      Dc = m2_sub({n.d0, n.d2, n.d2, n.d1}, m2_mul(Nm, m2_t(Ri)));
       double c0, c1;
       m2_mv(Nm, b0, b1, c0, c1);
-      b0 = B0[q] - c0;
-      b1 = B1[q] - c1;
+      b0 = n.b0 - c0;
+      b1 = n.b1 - c1;
       S = m2_neg(m2_mul(Nm, S));
+      n = nx;
     }
     const M2 Di = m2_inv(Dc);
     const M2 uL = m2_neg(m2_mul(Di, La)), uR = m2_neg(m2_mul(Di, S));
     double u0, u1;
     m2_mv(Di, b0, b1, u0, u1);
-    double* r = red + (size_t)blockDim.x * kCrStride + (size_t)t * kRelStride;
+    double* r = rel + (size_t)tid * kRelStride;
     r[0] = uL.a; r[1] = uL.b; r[2] = uL.c; r[3] = uL.d;
     r[4] = uR.a; r[5] = uR.b; r[6] = uR.c; r[7] = uR.d;
     r[8] = u0; r[9] = u1;
@@ -205,31 +234,35 @@ __device__ void part_solve(double* pl, int h, double* red, double* xo, int xs, d
   double u0e = 0, u1e = 0;
   if (own && mt >= 2) {
     size_t q = L.pos(t, 0);
-    M2 Di = m2_inv({D0[q], D2[q], D2[q], D1[q]});
-    double b0 = B0[q], b1 = B1[q];
+    Node n = ldN(0);
+    M2 Di = m2_inv({n.d0, n.d2, n.d2, n.d1});
+    double b0 = n.b0, b1 = n.b1;
     M2 S = La;
-    M2 Rp = ldR(q);
+    M2 Rp = n.R;
+    if (mt >= 3) n = ldN(1);
     for (int k = 0;; k++) {
       D0[q] = Di.a; D1[q] = Di.d; D2[q] = 0.5 * (Di.b + Di.c);
       S0[q] = S.a; S1[q] = S.b; S2[q] = S.c; S3[q] = S.d;
       B0[q] = b0; B1[q] = b1;
       if (k + 1 >= mt - 1) break;
       q = L.pos(t, k + 1);
+      const Node nx = k + 2 < mt - 1 ? ldN(k + 2) : n;
       const M2 M = m2_mul(m2_t(Rp), Di);  // L_{i+1} D~_i^-1 with L_{i+1} = R_i^T
-      Di = m2_inv(m2_sub({D0[q], D2[q], D2[q], D1[q]}, m2_mul(M, Rp)));
+      Di = m2_inv(m2_sub({n.d0, n.d2, n.d2, n.d1}, m2_mul(M, Rp)));
       double c0, c1;
       m2_mv(M, b0, b1, c0, c1);
-      b0 = B0[q] - c0;
-      b1 = B1[q] - c1;
+      b0 = n.b0 - c0;
+      b1 = n.b1 - c1;
       S = m2_neg(m2_mul(M, S));
-      Rp = ldR(q);
+      Rp = n.R;
+      n = nx;
     }
     // Rp = R_{e-1}, Di = D~_{e-1}^-1
     uRe = m2_neg(m2_mul(Di, Rp));
     uLe = m2_neg(m2_mul(Di, S));
     m2_mv(Di, b0, b1, u0e, u1e);
   }
-  __syncthreads();
+  cluster.sync();
   // separator rows of the reduced system
   if (own) {
     const size_t qe = L.pos(t, mt - 1);
@@ -251,7 +284,8 @@ __device__ void part_solve(double* pl, int h, double* red, double* xo, int xs, d
     }
     if (t + 1 < P) {
       if (L.m(t + 1) >= 2) {
-        const double* w = red + (size_t)blockDim.x * kCrStride + (size_t)(t + 1) * kRelStride;
+        const double* w = tid + 1 < bd ? rel + (size_t)(tid + 1) * kRelStride
+                                       : cluster.map_shared_rank(rel, (unsigned)cluster.block_rank() + 1);
         const M2 uL1 = {w[0], w[1], w[2], w[3]}, uR1 = {w[4], w[5], w[6], w[7]};
         Dr = m2_add(Dr, m2_mul(Re, uL1));
         Rr = m2_mul(Re, uR1);
@@ -262,45 +296,65 @@ __device__ void part_solve(double* pl, int h, double* red, double* xo, int xs, d
         Rr = Re;
       }
     }
-    double* r = red + (size_t)t * kCrStride;
+    double* r = red + (size_t)tid * kCrStride;
     r[0] = Dr.a; r[1] = Dr.d; r[2] = 0.5 * (Dr.b + Dr.c);
     r[3] = Lr.a; r[4] = Lr.b; r[5] = Lr.c; r[6] = Lr.d;
     r[7] = Rr.a; r[8] = Rr.b; r[9] = Rr.c; r[10] = Rr.d;
     r[11] = b0; r[12] = b1;
   }
-  __syncthreads();
-  cr_solve(red, P);
+  cluster.sync();
+  cr_solve(cluster, red, P);
   // back substitution of the interior
   if (own) {
-    const double xl0 = t > 0 ? red[(size_t)(t - 1) * kCrStride + 11] : 0.0;
-    const double xl1 = t > 0 ? red[(size_t)(t - 1) * kCrStride + 12] : 0.0;
-    double x0 = red[(size_t)t * kCrStride + 11], x1 = red[(size_t)t * kCrStride + 12];
+    double xl0 = 0.0, xl1 = 0.0;
+    if (t > 0) {
+      const double* w = tid > 0 ? red + (size_t)(tid - 1) * kCrStride
+                                : cluster.map_shared_rank(red, (unsigned)cluster.block_rank() - 1) +
+                                      (size_t)(bd - 1) * kCrStride;
+      xl0 = w[11];
+      xl1 = w[12];
+    }
+    double x0 = red[(size_t)tid * kCrStride + 11], x1 = red[(size_t)tid * kCrStride + 12];
     xo[(size_t)e * xs] = x0;
     yo[(size_t)e * ys] = x1;
-    for (int k = mt - 2; k >= 0; k--) {
+    struct Back {
+      Node n;
+      M2 S;
+    };
+    auto ldB = [&](int k) -> Back {
       const size_t q = L.pos(t, k);
-      const M2 Di = {D0[q], D2[q], D2[q], D1[q]};
+      return {ldN(k), {S0[q], S1[q], S2[q], S3[q]}};
+    };
+    Back w = mt >= 2 ? ldB(mt - 2) : Back{};
+    for (int k = mt - 2; k >= 0; k--) {
+      const Back nx = k > 0 ? ldB(k - 1) : w;
+      const M2 Di = {w.n.d0, w.n.d2, w.n.d2, w.n.d1};
       double c0, c1, s0, s1;
-      m2_mv({S0[q], S1[q], S2[q], S3[q]}, xl0, xl1, s0, s1);
-      m2_mv(ldR(q), x0, x1, c0, c1);  // R_i x_{i+1}
-      m2_mv(Di, B0[q] - s0 - c0, B1[q] - s1 - c1, x0, x1);
+      m2_mv(w.S, xl0, xl1, s0, s1);
+      m2_mv(w.n.R, x0, x1, c0, c1);  // R_i x_{i+1}
+      m2_mv(Di, w.n.b0 - s0 - c0, w.n.b1 - s1 - c1, x0, x1);
       xo[(size_t)(a + k) * xs] = x0;
       yo[(size_t)(a + k) * ys] = x1;
+      w = nx;
     }
   }
-  __syncthreads();
+  cluster.sync();
 }
 
 // Standalone solve of a block-tridiagonal system given as diag (n x 3: xx yy xy), coupling
 // ((n-1) x 4: [[c0 c2] [c3 c1]] between block i and i+1) and rhs (n x 2) into x (n x 2), with
-// the caller's workspace cr (n x kCrStride doubles). One CTA with blockDim.x x kPartSmemStride
-// doubles of dynamic shared memory.
-__global__ void __launch_bounds__(kSolveThreads) k_block_tridiag(int n, const double* __restrict__ diag,
-                                                                 const double* __restrict__ coupling,
-                                                                 const double* __restrict__ rhs,
-                                                                 double* __restrict__ x, double* __restrict__ cr) {
-  const PartLayout L(n, blockDim.x);
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+// the caller's workspace cr (n x kCrStride doubles). One cluster of kTridiagThreads-thread CTAs with
+// kTridiagThreads x kPartSmemStride doubles of dynamic shared memory each: twice the partitions of
+// the half-step solve (8 nodes a partition at 16385).
+constexpr int kTridiagThreads = 256;
+__global__ void __cluster_dims__(kSolveCluster, 1, 1) __launch_bounds__(kTridiagThreads)
+    k_block_tridiag(int n, const double* __restrict__ diag, const double* __restrict__ coupling,
+                    const double* __restrict__ rhs, double* __restrict__ x, double* __restrict__ cr) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int ranks = solve_ranks(n), rank = (int)cluster.block_rank();
+  if (rank >= ranks) return;
+  const PartLayout L(n, kTridiagThreads * kSolveCluster);
+  for (int i = rank * blockDim.x + threadIdx.x; i < n; i += ranks * blockDim.x) {
     const size_t q = L.pos_of(i);
     cr[(size_t)kPD0 * n + q] = diag[3 * i];
     cr[(size_t)kPD1 * n + q] = diag[3 * i + 1];
@@ -314,9 +368,9 @@ __global__ void __launch_bounds__(kSolveThreads) k_block_tridiag(int n, const do
     cr[(size_t)kPB0 * n + q] = rhs[2 * i];
     cr[(size_t)kPB1 * n + q] = rhs[2 * i + 1];
   }
-  __syncthreads();
+  cluster.sync();
   extern __shared__ double sh_red[];  // blockDim.x x kPartSmemStride
-  part_solve(cr, n, sh_red, x, 2, x + 1, 2);
+  part_solve(cluster, cr, n, sh_red, x, 2, x + 1, 2);
 }
 
 // Knot-difference regulariser of frame f (extension; lambda = 0 reproduces the reference): sum of
@@ -333,10 +387,13 @@ __device__ inline double frame_reg_warp(const double* own, int W, int N, double 
 }
 
 // Chunked scan of SmearingFilter::apply (smearingfilter.cpp:24-33), v_i = s v_{i-1} + (1-s) v_i with
-// v_{-1} = 0, over n values. Each thread runs the exact recurrence on its chunk from a carry-in that
-// composes the preceding chunks' affine maps.
-__device__ void smear_scan(double* v, int n, double s, double* sh_a, double* sh_b) {
-  const int nt = blockDim.x, t = threadIdx.x;
+// v_{-1} = 0, over n values with the first `ranks` CTAs of a cluster (kSolveThreads threads in all, the
+// chunks of the CTAs past `ranks` being empty). Each thread runs the exact recurrence on its chunk from
+// a carry-in that composes the preceding chunks' affine maps. sh: 3 doubles per warp of this CTA.
+__device__ void smear_scan(cg::cluster_group& cluster, int ranks, double* v, int n, double s, double* sh) {
+  const int nt = kSolveThreads, rank = (int)cluster.block_rank(), wpc = blockDim.x >> 5;
+  const int t = rank * blockDim.x + threadIdx.x;
+  double *sh_a = sh, *sh_b = sh + wpc, *sh_c = sh + 2 * wpc;
   const int chunk = (n + nt - 1) / nt;
   const int lo = min(n, t * chunk), hi = min(n, lo + chunk);
   const double om = 1.0 - s;
@@ -347,7 +404,8 @@ __device__ void smear_scan(double* v, int n, double s, double* sh_a, double* sh_
   }
   // carry-in of each chunk: exclusive scan of the chunks' affine maps c -> a c + y (composition
   // (a2, b2) after (a1, b1) = (a2 a1, a2 b1 + b2)), warp scans then a scan of the warp totals
-  const int lane = t & 31, warp = t >> 5, nw = (nt + 31) >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  static_assert(kSolveThreads == 32 * 32, "one lane per warp of the cluster");
   double A = a, B = y;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -361,9 +419,11 @@ __device__ void smear_scan(double* v, int n, double s, double* sh_a, double* sh_
     sh_a[warp] = A;
     sh_b[warp] = B;
   }
-  __syncthreads();
-  if (warp == 0) {
-    double wa = lane < nw ? sh_a[lane] : 1.0, wb = lane < nw ? sh_b[lane] : 0.0;
+  cluster.sync();
+  if (warp == 0) {  // every CTA scans the totals of all warps
+    const int q = lane / wpc;
+    double wa = q < ranks ? cluster.map_shared_rank(sh_a, q)[lane - q * wpc] : 1.0;
+    double wb = q < ranks ? cluster.map_shared_rank(sh_b, q)[lane - q * wpc] : 0.0;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const double pa = __shfl_up_sync(0xffffffffu, wa, o), pb = __shfl_up_sync(0xffffffffu, wb, o);
@@ -374,22 +434,20 @@ __device__ void smear_scan(double* v, int n, double s, double* sh_a, double* sh_
     }
     // exclusive: the composition of the preceding warps applied to 0
     const double ex = __shfl_up_sync(0xffffffffu, wb, 1);
-    __syncwarp();
-    if (lane < nw) sh_b[32 + lane] = lane == 0 ? 0.0 : ex;
+    if (q == rank) sh_c[lane - q * wpc] = lane == 0 ? 0.0 : ex;
   }
   __syncthreads();
   {
     // this thread's exclusive in-warp map applied to the warp's carry-in
     const double ea = __shfl_up_sync(0xffffffffu, A, 1), eb = __shfl_up_sync(0xffffffffu, B, 1);
-    const double cw = sh_b[32 + warp];
+    const double cw = sh_c[warp];
     y = lane == 0 ? cw : ea * cw + eb;
   }
-  __syncthreads();
   for (int i = lo; i < hi; i++) {
     y = __dadd_rn(__dmul_rn(y, s), __dmul_rn(v[i], om));
     v[i] = y;
   }
-  __syncthreads();
+  cluster.sync();  // v is complete, and the totals are free for the next call
 }
 
 // RangeFilter::apply (rangefilter.cpp:24-40): a sequential, data-dependent recurrence.
@@ -408,8 +466,8 @@ __device__ void range_seq(double* v, int n, double strength) {
 // The half-step solve of every group in phase kPhHalf runs as five launches: the per-column and
 // per-frame set-up and the block assembly are spread over kSolveSplit CTAs per group
 // (k_solve_prep, k_solve_planes, k_solve_expand), the steps that need the whole group in one CTA
-// (compaction, the partitioned solve and the filters) run one 1024-thread CTA per group
-// (k_solve_compact, k_solve_system). A single CTA per group spent most of its time in the
+// (compaction; the partitioned solve and the filters) run one 1024-thread CTA (k_solve_compact) or one
+// cluster (k_solve_system) per group. A single CTA per group spent most of its time in the
 // independent per-node work, bound by one SM's global-memory queue.
 //   blocksPresent / paramsUsed / errval (task_applyparameters.cuh:74-81, task_createparametermask.cuh,
 //   task_calcerrval.cu:185), the filter switch-off (mainiteration.cpp:246-256), compaction
@@ -763,41 +821,44 @@ __device__ void ilu0_solve_seq(const double* __restrict__ pl, int h, const int* 
   }
 }
 
-// The partitioned FP64 solve, the solver's filter and the median of flag R (one CTA per group).
-__global__ void __launch_bounds__(kSolveThreads) k_solve_system(const GroupDesc* __restrict__ gds,
-                                                                GroupCtl* __restrict__ ctl) {
-  const GroupDesc& G = gds[blockIdx.x];
-  GroupCtl& C = ctl[blockIdx.x];
+// The partitioned FP64 solve, the solver's filter and the median of flag R: a cluster of kSolveCluster
+// CTAs per group, of which solve_ranks take part.
+__global__ void __cluster_dims__(kSolveCluster, 1, 1) __launch_bounds__(kSolveSysThreads)
+    k_solve_system(const GroupDesc* __restrict__ gds, GroupCtl* __restrict__ ctl) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const GroupDesc& G = gds[blockIdx.x / kSolveCluster];
+  GroupCtl& C = ctl[blockIdx.x / kSolveCluster];
   if (!C.solve_now) return;
-  const int t = threadIdx.x, nt = blockDim.x;
-  const int h = C.n_used >> 1;
-  __shared__ double sh_a[kSolveThreads], sh_b[kSolveThreads];
+  const int h = C.n_used >> 1, rank = (int)cluster.block_rank();
+  const int ranks = solve_ranks(h);
+  if (rank >= ranks) return;
+  const int t = rank * blockDim.x + threadIdx.x, nt = ranks * blockDim.x;
 
   // (4) FP64 solve into the compact step [x_0..x_h-1, y_0..y_h-1]: ILU(0) for solver id 0, else the
   // exact partitioned block-tridiagonal solve
-  extern __shared__ double sh_red[];  // kSolveThreads x kPartSmemStride
+  extern __shared__ double sh_red[];  // kSolveSysThreads x kPartSmemStride
   if (G.solver_id == 0) {
     if (t == 0 && h > 0) ilu0_solve_seq(G.cr, h, G.list, G.ilu, G.ndp, G.ndp + h);
-    __syncthreads();
+    cluster.sync();
   } else {
-    part_solve(G.cr, h, sh_red, G.ndp, 1, G.ndp + h, 1);
+    part_solve(cluster, G.cr, h, sh_red, G.ndp, 1, G.ndp + h, 1);
   }
   // (6) the solver's filter on the x half and the y half (eigensolver.cu:54-55)
   if (C.filter_active) {
     if (C.filter_kind == 1) {
-      smear_scan(G.ndp, h, G.filter_strength, sh_a, sh_b);
-      smear_scan(G.ndp + h, h, G.filter_strength, sh_a, sh_b);
+      smear_scan(cluster, ranks, G.ndp, h, G.filter_strength, sh_red);
+      smear_scan(cluster, ranks, G.ndp + h, h, G.filter_strength, sh_red);
     } else {
       if (t == 0) range_seq(G.ndp, h, G.filter_strength);
       if (t == 32) range_seq(G.ndp + h, h, G.filter_strength);
-      __syncthreads();
+      cluster.sync();
     }
   }
   // (7) 3-tap median of each half (flag R), out of place, ends kept
   if (G.flags & kFlagMedianBefore) {
     double* tmp = G.cr;  // free after the solve
     for (int i = t; i < 2 * h; i += nt) tmp[i] = G.ndp[i];
-    __syncthreads();
+    cluster.sync();
     for (int i = t; i < 2 * h; i += nt) {
       int base = i < h ? 0 : h, j = i - base;
       if (j == 0 || j == h - 1) continue;
@@ -805,7 +866,6 @@ __global__ void __launch_bounds__(kSolveThreads) k_solve_system(const GroupDesc*
       int k = 1 * ((b >= a && b < c) || (b <= a && b > c)) + 2 * ((c >= a && c < b) || (c >= b && c < a));
       G.ndp[i] = k == 0 ? a : (k == 1 ? b : c);
     }
-    __syncthreads();
   }
 }
 
