@@ -2661,7 +2661,14 @@ int reconstruct_frames(const ss_reconstruct* r) {
   if (r->gpu_device_id < 0 || r->gpu_device_id >= ndev) return fail(SS_ERR_INVALID_ARGUMENT, "gpu_device_id out of range");
   SS_CK(cudaSetDevice(r->gpu_device_id));
 
-  const int chunk = std::min(n, 64);
+  // Iterates kept per frame (slot 0, the first guess, and a ring of the later ones): 64 where 64 frames of
+  // them fit in kRingBytes (a 512 x 512 frame takes 64 MB), so that a set's outputs are at hand when its
+  // stops are known; larger frames run fewer at a time, and the largest with a shorter ring.
+  constexpr size_t kRingBytes = size_t(4) << 30;
+  const int rh = (th + 1) / 2, cw = (tw + 1) / 2;
+  const size_t iterate = 16 * (size_t)rh * cw;  // bytes
+  const int slots = (int)std::min<size_t>(64, std::max<size_t>(kRcBatch + 2, kRingBytes / iterate));
+  const int chunk = (int)std::max<size_t>(1, std::min<size_t>({(size_t)n, (size_t)64, kRingBytes / (iterate * slots)}));
   const size_t px = (size_t)hd * wd, fsz = fr.dtype == SS_F64 ? 8 : 4, osz = o.dtype == SS_F64 ? 8 : 4;
   CallMem m;
   SS_CK(cudaStreamCreateWithFlags(&m.s, cudaStreamNonBlocking));
@@ -2685,6 +2692,10 @@ int reconstruct_frames(const ss_reconstruct* r) {
   b.hd = (int)hd;
   b.wd = (int)wd;
   b.nk = nk;
+  b.rh = rh;
+  b.cw = cw;
+  b.nq = rh * cw;
+  b.frames = chunk;
   const size_t cnp = (size_t)chunk * np;
   b.wy = m.take<double>(cnp);
   b.ww = m.take<double>(cnp * kRcStencil);
@@ -2693,25 +2704,21 @@ int reconstruct_frames(const ss_reconstruct* r) {
   b.last_z = m.take<int>(cnp);
   b.last_n = m.take<int>(cnp);
   b.mask = m.take<uint8_t>(cnp);
-  b.coef = m.take<float>(cnp * 10);
+  b.coef = m.take<float>((size_t)chunk * kRcTerms * 4 * b.nq);
   b.le = m.take<float>(cnp);
-  b.x = m.take<float>(cnp);
-  b.xo = m.take<float>(cnp);
-  b.part = m.take<double>((size_t)chunk * kRcParts);
-  b.part_l = m.take<float>((size_t)chunk * kRcParts);
-  int* d_state = m.take<int>(chunk);
-  int* d_due = m.take<int>(chunk);
-  int* d_keep = m.take<int>(chunk);
-  int* d_iters = m.take<int>(chunk);
-  int* d_interval = m.take<int>(chunk);
+  b.x = m.take<float>((size_t)slots * chunk * 4 * b.nq);
+  b.part = m.take<double>((size_t)chunk * kRcParts * kRcBatch);
+  b.part_l = m.take<float>((size_t)chunk * kRcParts * kRcBatch);
+  int* d_limit = m.take<int>(chunk);
   int* d_count = m.take<int>(chunk);
   int* d_skip = m.take<int>(chunk);
-  float* d_eo = m.take<float>(chunk);
+  int* d_slot = m.take<int>(chunk);
+  float* d_energy = m.take<float>((size_t)chunk * kRcBatch);
   void* d_out = o.location == SS_DEVICE ? const_cast<void*>(o.data) : m.take<char>(osz * cnp);
   uint8_t* d_mk = r->mask ? m.take<uint8_t>(cnp) : nullptr;
   if (!d_bx || !d_by || !d_tf || !d_pk || !d_dxk || !d_dyk || !d_data || !b.wy || !b.ww || !b.z || !b.cnt ||
-      !b.last_z || !b.last_n || !b.mask || !b.coef || !b.le || !b.x || !b.xo || !b.part || !b.part_l || !d_state ||
-      !d_due || !d_keep || !d_iters || !d_interval || !d_count || !d_skip || !d_eo || !d_out || (r->mask && !d_mk))
+      !b.last_z || !b.last_n || !b.mask || !b.coef || !b.le || !b.x || !b.part || !b.part_l || !d_limit || !d_count ||
+      !d_skip || !d_slot || !d_energy || !d_out || (r->mask && !d_mk))
     return fail(SS_ERR_OUT_OF_MEMORY, "reconstruct: work memory");
   SS_CK(cudaMemcpyAsync(d_bx, bx.data(), px * 8, cudaMemcpyHostToDevice, s));
   SS_CK(cudaMemcpyAsync(d_by, by.data(), px * 8, cudaMemcpyHostToDevice, s));
@@ -2722,125 +2729,137 @@ int reconstruct_frames(const ss_reconstruct* r) {
   const double regfac = r->regfac, vfac = 1.0 / r->pixel_aspect_ratio, vf2 = vfac * vfac;
   const int g = 148 * 8;
 
-  // Frames [a, a + nf) of the set with check intervals iv[0..nf): their sweeps to completion, their
-  // outputs into the chunk slots 0..nf; per-frame sweep counts (0: skipped) into it_out.
-  auto run = [&](int a, int nf, const std::vector<int>& iv, std::vector<int>& it_out) -> int {
-    const size_t fnp = (size_t)nf * np;
+  // Slot of iterate `it` (0: the first guess).
+  auto slot_of = [&](int it) { return it == 0 ? 0 : 1 + (it - 1) % (slots - 1); };
+  auto sweep = [&](int nf, int it) {
+    const dim3 fg(std::max(1, g / nf), nf);  // at most g CTAs (one wave) over the frames
+    const int so = slot_of(it - 1), sn = slot_of(it);
+    k_rc_sweep<0><<<fg, 256, 0, s>>>(b, it, so, sn, d_limit);
+    k_rc_sweep<1><<<fg, 256, 0, s>>>(b, it, so, sn, d_limit);
+    k_rc_sweep<2><<<fg, 256, 0, s>>>(b, it, so, sn, d_limit);
+    k_rc_sweep<3><<<fg, 256, 0, s>>>(b, it, so, sn, d_limit);
+  };
+  auto energies = [&](int nf, int it0, int nit) {
+    const int4 sl = make_int4(slot_of(it0), slot_of(it0 + 1), slot_of(it0 + 2), slot_of(it0 + 3));
+    k_rc_linear<<<dim3(kRcParts, nf), 256, 0, s>>>(b, it0, nit, sl, d_limit);
+    k_rc_quadratic<<<dim3(kRcParts, nf), 256, 0, s>>>(b, it0, nit, sl, d_limit, regfac, vf2);
+    k_rc_total<<<(nf * kRcBatch + 127) / 128, 128, 0, s>>>(b, nf, it0, nit, d_limit, d_energy);
+  };
+  constexpr int kIntervals = 10;     // rc_interval is 1..10
+  constexpr int kMaxSweeps = 1 << 22;
+
+  int carried = 1;  // the interval entering the next frame; 1 at the start of a call
+  for (int f0 = 0; f0 < n; f0 += chunk) {
+    const int F = std::min(chunk, n - f0);
+    const size_t fnp = (size_t)F * np;
     SS_CK(cudaMemsetAsync(b.wy, 0, fnp * 8, s));
     SS_CK(cudaMemsetAsync(b.ww, 0, fnp * kRcStencil * 8, s));
     SS_CK(cudaMemsetAsync(b.z, 0, fnp * 4, s));
     SS_CK(cudaMemsetAsync(b.cnt, 0, fnp * 4, s));
-    SS_CK(cudaMemsetAsync(d_count, 0, nf * 4, s));
-    SS_CK(cudaMemsetAsync(d_iters, 0, nf * 4, s));
+    SS_CK(cudaMemsetAsync(d_count, 0, F * 4, s));
     if (fr.dtype == SS_F64)
-      k_rc_constraints<double><<<g, 256, 0, s>>>(b, d_data, a, nf, d_bx, d_by, d_tf, d_pk, d_dxk, d_dyk);
+      k_rc_constraints<double><<<g, 256, 0, s>>>(b, d_data, f0, F, d_bx, d_by, d_tf, d_pk, d_dxk, d_dyk);
     else
-      k_rc_constraints<float><<<g, 256, 0, s>>>(b, d_data, a, nf, d_bx, d_by, d_tf, d_pk, d_dxk, d_dyk);
+      k_rc_constraints<float><<<g, 256, 0, s>>>(b, d_data, f0, F, d_bx, d_by, d_tf, d_pk, d_dxk, d_dyk);
     for (int st = 0; st < 4; st++) {
-      k_rc_fill_int<<<g, 256, 0, s>>>(b.last_z, fnp, -1);
-      k_rc_fill_int<<<g, 256, 0, s>>>(b.last_n, fnp, -1);
+      SS_CK(cudaMemsetAsync(b.last_z, 0xFF, fnp * 4, s));  // -1
+      SS_CK(cudaMemsetAsync(b.last_n, 0xFF, fnp * 4, s));
       for (int ph = 0; ph < 2; ph++) {
         if (fr.dtype == SS_F64)
-          k_rc_pushgrid<double><<<g, 256, 0, s>>>(b, d_data, a, nf, st, ph, d_bx, d_by, d_tf, d_pk, d_dxk, d_dyk);
+          k_rc_pushgrid<double><<<g, 256, 0, s>>>(b, d_data, f0, F, st, ph, d_bx, d_by, d_tf, d_pk, d_dxk, d_dyk);
         else
-          k_rc_pushgrid<float><<<g, 256, 0, s>>>(b, d_data, a, nf, st, ph, d_bx, d_by, d_tf, d_pk, d_dxk, d_dyk);
+          k_rc_pushgrid<float><<<g, 256, 0, s>>>(b, d_data, f0, F, st, ph, d_bx, d_by, d_tf, d_pk, d_dxk, d_dyk);
       }
     }
-    k_rc_mask<<<g, 256, 0, s>>>(b, nf);
-    k_rc_coef<<<g, 256, 0, s>>>(b, nf, regfac, vf2);
-    const dim3 fg(std::max(1, g / nf), nf);  // per-frame grids: at most g CTAs (one wave) over the frames
-    k_rc_count<<<fg, 256, 0, s>>>(b, d_count);
+    k_rc_mask<<<g, 256, 0, s>>>(b, F);
+    k_rc_coef<<<g, 256, 0, s>>>(b, F, regfac, vf2);
+    k_rc_count<<<dim3(std::max(1, g / F), F), 256, 0, s>>>(b, d_count);
     SS_CK(cudaGetLastError());
-    std::vector<int> count(nf), state(nf), due(nf);
-    SS_CK(cudaMemcpyAsync(count.data(), d_count, nf * 4, cudaMemcpyDeviceToHost, s));
+    // the vectors below are the sources and targets of copies on s: each round waits for its copies
+    std::vector<int> count(F), limit(F), skip(F), slot(F, -1), iters(F, 0), swept(F, 0), target(F, 0);
+    std::vector<float> got((size_t)F * kRcBatch);
+    SS_CK(cudaMemcpyAsync(count.data(), d_count, F * 4, cudaMemcpyDeviceToHost, s));
     SS_CK(cudaStreamSynchronize(s));
-    int running = 0;
-    for (int f = 0; f < nf; f++) {
-      state[f] = count[f] > 0 ? 1 : 3;
-      due[f] = state[f] == 1;
-      running += due[f];
+    for (int f = 0; f < F; f++) {
+      skip[f] = count[f] == 0;
+      limit[f] = skip[f] ? -1 : INT_MAX;
     }
-    SS_CK(cudaMemcpyAsync(d_state, state.data(), nf * 4, cudaMemcpyHostToDevice, s));
-    SS_CK(cudaMemcpyAsync(d_due, due.data(), nf * 4, cudaMemcpyHostToDevice, s));
-    SS_CK(cudaMemcpyAsync(d_interval, iv.data(), nf * 4, cudaMemcpyHostToDevice, s));
-    std::vector<int> skip(nf);
-    for (int f = 0; f < nf; f++) skip[f] = state[f] == 3;
-    SS_CK(cudaMemcpyAsync(d_skip, skip.data(), nf * 4, cudaMemcpyHostToDevice, s));
-    const dim3 eg(kRcParts, nf);
-    const int cb = (nf + 127) / 128;
-    k_rc_energy<<<eg, 256, 0, s>>>(b, nf, d_due, regfac, vf2);
-    k_rc_check<<<cb, 128, 0, s>>>(nf, d_due, d_state, d_eo, d_keep, b.part, b.part_l, 1, 0, d_iters);
-    const int kMaxSweeps = 1 << 22;
-    for (int it = 1; running > 0; it++) {
-      if (it > kMaxSweeps) return fail(SS_ERR_CUDA, "reconstruct: the energy kept decreasing over 4M sweeps");
-      for (int colour = 0; colour < 4; colour++) k_rc_sweep<<<fg, 256, 0, s>>>(b, colour, d_state);
-      k_rc_due<<<cb, 128, 0, s>>>(nf, d_state, d_interval, it, d_due);
-      k_rc_energy<<<eg, 256, 0, s>>>(b, nf, d_due, regfac, vf2);
-      k_rc_check<<<cb, 128, 0, s>>>(nf, d_due, d_state, d_eo, d_keep, b.part, b.part_l, 0, it, d_iters);
-      k_rc_keep<<<fg, 256, 0, s>>>(b, d_keep);
-      if (it % 8 == 0) {
-        SS_CK(cudaMemcpyAsync(state.data(), d_state, nf * 4, cudaMemcpyDeviceToHost, s));
-        SS_CK(cudaStreamSynchronize(s));
-        running = 0;
-        for (int f = 0; f < nf; f++) running += state[f] == 1;
-      }
-    }
-    SS_CK(cudaGetLastError());
-    it_out.resize(nf);
-    SS_CK(cudaMemcpyAsync(it_out.data(), d_iters, nf * 4, cudaMemcpyDeviceToHost, s));
-    char* dst = o.location == SS_DEVICE ? static_cast<char*>(d_out) + osz * (size_t)a * np : static_cast<char*>(d_out);
-    if (o.dtype == SS_F64) k_rc_out<double><<<g, 256, 0, s>>>(b, nf, (double*)dst, d_mk, d_skip);
-    else k_rc_out<float><<<g, 256, 0, s>>>(b, nf, (float*)dst, d_mk, d_skip);
-    SS_CK(cudaStreamSynchronize(s));
-    return SS_OK;
-  };
+    SS_CK(cudaMemcpyAsync(d_skip, skip.data(), F * 4, cudaMemcpyHostToDevice, s));
 
-  int carried = 1;  // the interval entering the next frame; 1 at the start of a call
-  std::vector<int> last_iters;
-  for (int f0 = 0; f0 < n; f0 += chunk) {
-    const int F = std::min(chunk, n - f0);
-    std::vector<int> guess(F, 10), iters(F, 0);
-    guess[0] = carried;
-    int start = 0;
-    while (start < F) {
-      std::vector<int> iv(guess.begin() + start, guess.end()), got;
-      int rc = run(f0 + start, F - start, iv, got);
-      if (rc) return rc;
-      // the chain of intervals from `start`: frames up to the first mismatch ran with their own
-      int cur = guess[start], bad = -1;
-      for (int i = start; i < F; i++) {
-        if (guess[i] != cur) {
-          bad = i;
-          break;
+    // energies of the last 16 iterates, and the stop of each interval (0: not yet)
+    struct Trace {
+      float e[16];
+      int stop[kIntervals + 1] = {};
+      int open = kIntervals;
+    };
+    std::vector<Trace> trace(F);
+    int next = 0, cur = carried;  // frames below `next` are settled; cur: the interval entering frame next
+    auto settle = [&] {
+      for (; next < F; next++) {
+        if (skip[next]) continue;  // skipped frames keep the interval
+        const int st = trace[next].stop[cur];
+        if (!st) return;
+        iters[next] = st;
+        target[next] = st - cur;
+        cur = rc_interval(st);
+      }
+    };
+    settle();
+    for (int it = 0; next < F; it += it ? kRcBatch : 1) {  // iterate 0, then kRcBatch at a time
+      if (it > kMaxSweeps) return fail(SS_ERR_CUDA, "reconstruct: the energy kept decreasing over 4M sweeps");
+      const int nit = it ? kRcBatch : 1;
+      SS_CK(cudaMemcpyAsync(d_limit, limit.data(), F * 4, cudaMemcpyHostToDevice, s));
+      if (it)
+        for (int k = 0; k < nit; k++) sweep(F, it + k);
+      energies(F, it, nit);
+      SS_CK(cudaGetLastError());
+      SS_CK(cudaMemcpyAsync(got.data(), d_energy, got.size() * 4, cudaMemcpyDeviceToHost, s));
+      SS_CK(cudaStreamSynchronize(s));
+      for (int f = 0; f < F; f++) {
+        if (limit[f] < 0) continue;
+        Trace& t = trace[f];
+        for (int k = 0; k < nit; k++) {
+          const int i = it + k;
+          t.e[i & 15] = got[(size_t)f * kRcBatch + k];
+          for (int iv = 1; i > 0 && iv <= kIntervals; iv++)
+            if (!t.stop[iv] && i % iv == 0 && t.e[(i - iv) & 15] <= t.e[i & 15]) {
+              t.stop[iv] = i;
+              t.open--;
+            }
         }
-        iters[i] = got[i - start];
-        if (iters[i] > 0) cur = rc_interval(iters[i]);  // skipped frames keep the interval
+        swept[f] = it + nit - 1;
       }
-      const int good_end = bad < 0 ? F : bad;
-      // outputs of the settled frames [start, good_end) to the host
-      if (o.location == SS_HOST && good_end > start)
-        SS_CK(cudaMemcpy(static_cast<char*>(const_cast<void*>(o.data)) + osz * (size_t)(f0 + start) * np,
-                         d_out, osz * (size_t)(good_end - start) * np, cudaMemcpyDeviceToHost));
-      if (r->mask && good_end > start)
-        SS_CK(cudaMemcpy(r->mask + (size_t)(f0 + start) * np, d_mk, (size_t)(good_end - start) * np,
-                         cudaMemcpyDeviceToHost));
-      if (bad < 0) {
-        carried = cur;
-        break;
-      }
-      // re-run from the first frame that ran with another interval, with the intervals this run's
-      // sweep counts give (its own is now exact)
-      guess[bad] = cur;
-      int g2 = cur;
-      for (int i = bad + 1; i < F; i++) {
-        const int prev = got[i - 1 - start];
-        if (prev > 0) g2 = rc_interval(prev);
-        guess[i] = g2;
-      }
-      start = bad;
+      settle();
+      for (int f = 0; f < F; f++)
+        if (f < next || trace[f].open == 0) limit[f] = -1;
     }
-    if (r->iterations)
-      for (int i = 0; i < F; i++) r->iterations[f0 + i] = iters[i];
+    carried = cur;
+    // the outputs' iterates: still in the ring, or swept again from the first guess
+    int again = 0;
+    for (int f = 0; f < F; f++) {
+      limit[f] = -1;
+      if (skip[f] || target[f] == 0) continue;
+      slot[f] = slot_of(target[f]);
+      if (target[f] <= swept[f] - (slots - 1)) {
+        limit[f] = target[f];
+        again = std::max(again, target[f]);
+      }
+    }
+    if (again) {
+      SS_CK(cudaMemcpyAsync(d_limit, limit.data(), F * 4, cudaMemcpyHostToDevice, s));
+      for (int it = 1; it <= again; it++) sweep(F, it);
+    }
+    SS_CK(cudaMemcpyAsync(d_slot, slot.data(), F * 4, cudaMemcpyHostToDevice, s));
+    char* dst = o.location == SS_DEVICE ? static_cast<char*>(d_out) + osz * (size_t)f0 * np : static_cast<char*>(d_out);
+    if (o.dtype == SS_F64) k_rc_out<double><<<g, 256, 0, s>>>(b, F, (double*)dst, d_mk, d_slot, d_skip);
+    else k_rc_out<float><<<g, 256, 0, s>>>(b, F, (float*)dst, d_mk, d_slot, d_skip);
+    SS_CK(cudaGetLastError());
+    if (o.location == SS_HOST)
+      SS_CK(cudaMemcpyAsync(static_cast<char*>(const_cast<void*>(o.data)) + osz * (size_t)f0 * np, d_out, osz * fnp,
+                            cudaMemcpyDeviceToHost, s));
+    if (r->mask) SS_CK(cudaMemcpyAsync(r->mask + (size_t)f0 * np, d_mk, fnp, cudaMemcpyDeviceToHost, s));
+    SS_CK(cudaStreamSynchronize(s));
+    if (r->iterations) std::copy(iters.begin(), iters.end(), r->iterations + f0);
   }
   return SS_OK;
 }

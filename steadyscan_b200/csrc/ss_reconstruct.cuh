@@ -24,8 +24,12 @@
 //    term, compared in FP32) stops the frame when it did not decrease, the output being the
 //    iterate of the last check that decreased it (zeros if none did); n is the interval the
 //    previous frame's sweep count gave (:391).
-// Frames run in parallel: the sweeps do not depend on n, and the host re-runs a frame whose
-// interval, recomputed from its predecessor's sweep count, differs from the one it ran with.
+// Frames run in parallel, once: the iterates do not depend on n, so every sweep of every frame is kept
+// as its own iterate (in a ring of slots) with its energy, and the host follows the chain of intervals
+// over the energies; a frame sweeps until its stop is known, or the stop of every interval 1..10 is.
+// Guessing the intervals and sweeping again from the first wrong guess took seven runs of a 64-frame
+// set and a separate copy of every kept iterate (64 frames of 512 x 512: 150 ms a call, 119 of them on
+// the device; here 44 and 20).
 #pragma once
 
 #include "ss_common.cuh"
@@ -34,24 +38,37 @@ namespace ss {
 
 constexpr int kRcStencil = 5;  // diagonal, S, NE, E, SE
 constexpr int kRcParts = 64;   // partial-sum CTAs per frame of the energy
+constexpr int kRcBatch = 4;    // iterates whose energies are summed by one launch
+constexpr int kRcTerms = 9;    // sweep coefficients of a pixel: Rmat[8], L
 
-// Per-frame buffers of a chunk of frames (device pointers; [frame * np + p] unless noted).
+// Per-frame buffers of a chunk of frames (device pointers; [frame * np + p] unless noted). What the
+// sweeps read lies colour by colour, so that a colour's lanes read consecutive floats: quarter plane
+// `colour` of rh x cw entries holds pixel (2 i + colour / 2, 2 j + colour % 2) at i + rh j.
 struct RcBufs {
   int th, tw, np, hd, wd, nk;  // template size, data frame size, knots per frame
+  int rh, cw, nq;   // quarter planes: ceil(th / 2) x ceil(tw / 2) = nq entries
+  int frames;       // frames of a slot
   double* wy;       // np
-  double* ww;       // np x kRcStencil, pixel-major
+  double* ww;       // kRcStencil planes of np
   float* z;         // np: push-grid sums, then the first guess
   float* cnt;       // np: push-grid weights
   int* last_z;      // np
   int* last_n;      // np
   uint8_t* mask;    // np
-  float* coef;      // np x 10: R, Rmat[8], L
+  float* coef;      // kRcTerms x 4 quarter planes
   float* le;        // np: single(Lfull) of masked pixels, else 0
-  float* x;         // np
-  float* xo;        // np
-  double* part;     // frames x kRcParts x 2: energy partial sums (FP64 quadratic, FP32-valued linear)
-  float* part_l;    // frames x kRcParts
+  float* x;         // [slot][frame] iterates of 4 quarter planes; slot 0 is the first guess
+  double* part;     // frames x kRcParts x kRcBatch: energy partial sums (FP64 quadratic, FP32 linear)
+  float* part_l;    // frames x kRcParts x kRcBatch
 };
+
+__device__ __forceinline__ float* rc_iterate(const RcBufs& b, int slot, int f) {
+  return b.x + ((size_t)slot * b.frames + f) * 4 * b.nq;
+}
+// Place of pixel (r, c) in an iterate.
+__device__ __forceinline__ size_t rc_place(const RcBufs& b, int r, int c) {
+  return (size_t)((r & 1) * 2 + (c & 1)) * b.nq + (r >> 1) + (size_t)b.rh * (c >> 1);
+}
 
 // Template coordinates of data pixel q (column-major in hd x wd) of frame f (steady_scan.m:452-453).
 __device__ __forceinline__ void rc_coords(const double* __restrict__ bx, const double* __restrict__ by,
@@ -87,14 +104,15 @@ __global__ void __launch_bounds__(256) k_rc_constraints(RcBufs b, const void* __
 #pragma unroll
     for (int c = 0; c < 4; c++) {
       atomicAdd(wy + pc[c], w[c] * d);
-      atomicAdd(ww + (size_t)pc[c] * kRcStencil + 0, w[c] * w[c]);
+      atomicAdd(ww + pc[c], w[c] * w[c]);
     }
-    atomicAdd(ww + (size_t)pc[0] * kRcStencil + 1, w[0] * w[1]);  // (y,x)-(y+1,x): S
-    atomicAdd(ww + (size_t)pc[2] * kRcStencil + 1, w[2] * w[3]);  // (y,x+1)-(y+1,x+1): S
-    atomicAdd(ww + (size_t)pc[0] * kRcStencil + 3, w[0] * w[2]);  // E
-    atomicAdd(ww + (size_t)pc[1] * kRcStencil + 3, w[1] * w[3]);  // E
-    atomicAdd(ww + (size_t)pc[0] * kRcStencil + 4, w[0] * w[3]);  // SE
-    atomicAdd(ww + (size_t)pc[1] * kRcStencil + 2, w[1] * w[2]);  // (y+1,x)-(y,x+1): NE
+    const size_t np = b.np;
+    atomicAdd(ww + 1 * np + pc[0], w[0] * w[1]);  // (y,x)-(y+1,x): S
+    atomicAdd(ww + 1 * np + pc[2], w[2] * w[3]);  // (y,x+1)-(y+1,x+1): S
+    atomicAdd(ww + 3 * np + pc[0], w[0] * w[2]);  // E
+    atomicAdd(ww + 3 * np + pc[1], w[1] * w[3]);  // E
+    atomicAdd(ww + 4 * np + pc[0], w[0] * w[3]);  // SE
+    atomicAdd(ww + 2 * np + pc[1], w[1] * w[2]);  // (y+1,x)-(y,x+1): NE
   }
 }
 
@@ -147,7 +165,7 @@ __device__ __forceinline__ double rc_ww(const double* __restrict__ ww, int th, i
   else if (d == th - 1) s = 2;
   else if (d == th) s = 3;
   else if (d == th + 1) s = 4;
-  return s < 0 ? 0.0 : ww[(size_t)lo * kRcStencil + s];
+  return s < 0 ? 0.0 : ww[(size_t)s * np + lo];
 }
 
 // Mask (column sums of ww > 0 and a finite first guess) and the first iterate of every pixel.
@@ -163,8 +181,7 @@ __global__ void __launch_bounds__(256) k_rc_mask(RcBufs b, int nf) {
     for (int j = 0; j < 9; j++) s += rc_ww(ww, th, b.np, p, nb[j]);
     const float iv = b.z[e] / b.cnt[e];
     b.mask[e] = (s > 0.0 && !isnan(iv)) ? 1 : 0;
-    b.x[e] = isnan(iv) ? 0.0f : iv;
-    b.xo[e] = 0.0f;
+    rc_iterate(b, 0, f)[rc_place(b, p % th, p / th)] = isnan(iv) ? 0.0f : iv;
   }
 }
 
@@ -186,7 +203,7 @@ __device__ __forceinline__ double rc_q(const RcBufs& b, const double* ww, const 
   return rc_ww(ww, th, b.np, p, q) + reg;
 }
 
-// FP32 coefficients of every pixel: R, the eight neighbour terms, L; and Le.
+// FP32 coefficients of every pixel: the eight neighbour terms and L; and Le.
 __global__ void __launch_bounds__(256) k_rc_coef(RcBufs b, int nf, double regfac, double vf2) {
   const size_t total = (size_t)b.np * nf;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
@@ -195,8 +212,9 @@ __global__ void __launch_bounds__(256) k_rc_coef(RcBufs b, int nf, double regfac
     const uint8_t* mk = b.mask + (size_t)f * b.np;
     const int th = b.th, np = b.np, i = p + 1;  // 1-based, as the finders
     const float R = (float)rc_q(b, ww, mk, p, p, regfac, vf2);
-    float* cf = b.coef + e * 10;
-    cf[0] = R;
+    // (the entries of a quarter plane past the template's last row or column are never read)
+    float* cf = b.coef + (size_t)f * kRcTerms * 4 * b.nq + rc_place(b, p % th, p / th);
+    const size_t plane = 4 * (size_t)b.nq;
     // N NE E SE S SW W NW (steady_scan.m:677-723), 1-based candidates and their bounds
     const int cand[8] = {i - 1, i + th - 1, i + th, i + th + 1, i + 1, i - th + 1, i - th, i - th - 1};
     const bool ok[8] = {(i - 1) % th != 0, ((i + th - 1) % th != 0) && (i + th - 1 < np), i + th <= np,
@@ -206,119 +224,180 @@ __global__ void __launch_bounds__(256) k_rc_coef(RcBufs b, int nf, double regfac
     for (int j = 0; j < 8; j++) {
       float t = 0.0f;
       if (R != 0.0f && ok[j]) t = (float)rc_q(b, ww, mk, p, cand[j] - 1, regfac, vf2) / R;
-      cf[1 + j] = t;
+      cf[j * plane] = t;
     }
     const float lf = mk[p] ? (float)b.wy[e] : 0.0f;
     float L = lf / R;
     if (!isfinite(L)) L = 0.0f;
-    cf[9] = L;
+    cf[8 * plane] = L;
     b.le[e] = lf;
   }
 }
 
-// One colour sweep of the frames still running (state[f] == 1).
-__global__ void __launch_bounds__(256) k_rc_sweep(RcBufs b, int colour, const int* __restrict__ state) {
+// One colour of one sweep, iterate `it` (slot `snew`) from its predecessor (slot `sold`), of the frames
+// that sweep that far (limit[f] >= it). A colour's eight neighbours are of the other colours: the ones
+// before it come from the new iterate, the ones after it from the old. Neighbours outside the template
+// have zero terms. Bound: HBM, 36 B of terms per pixel (pixel by pixel in memory, 10 floats each, a
+// colour of 64 frames of 512 x 512 took 48 us; colour by colour 42 us, 5.2 TB/s).
+template <int COLOUR>
+__global__ void __launch_bounds__(256) k_rc_sweep(RcBufs b, int it, int sold, int snew, const int* __restrict__ limit) {
   const int f = blockIdx.y;
-  if (state[f] != 1) return;
-  const int th = b.th, tw = b.tw;
-  const int rh = (th + 1 - (colour >> 1)) >> 1, cw = (tw + 1 - (colour & 1)) >> 1;  // rows / columns of the colour
-  const int per = rh * cw;
-  float* x = b.x + (size_t)f * b.np;
-  const float* cf0 = b.coef + (size_t)f * b.np * 10;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < per; k += gridDim.x * blockDim.x) {
-    const int r = 2 * (k % rh) + (colour >> 1), c = 2 * (k / rh) + (colour & 1);
-    const int p = r + th * c;
-    const float* cf = cf0 + (size_t)p * 10;
-    const int q[8] = {p - 1, p + th - 1, p + th, p + th + 1, p + 1, p - th + 1, p - th, p - th - 1};
+  if (limit[f] < it) return;
+  constexpr int pr = COLOUR >> 1, pc = COLOUR & 1;
+  // N NE E SE S SW W NW
+  constexpr int dr[8] = {-1, -1, 0, 1, 1, 1, 0, -1}, dc[8] = {0, 1, 1, 1, 0, -1, -1, -1};
+  const int th = b.th, tw = b.tw, rh = b.rh;
+  const size_t nq = b.nq;
+  const float* xo = rc_iterate(b, sold, f);
+  float* xn = rc_iterate(b, snew, f);
+  const float* cf = b.coef + (size_t)f * kRcTerms * 4 * nq + (size_t)COLOUR * nq;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < b.nq; k += gridDim.x * blockDim.x) {
+    const int j = k / rh, i = k - j * rh, r = 2 * i + pr, c = 2 * j + pc;
+    if (r >= th || c >= tw) continue;
+    float v[8], t[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      constexpr auto colour_of = [](int a, int e) { return (a & 1) * 2 + (e & 1); };
+      const int qc = colour_of(pr + dr[q] + 2, pc + dc[q] + 2);
+      const int qi = i + ((pr + dr[q] + 2) >> 1) - 1, qj = j + ((pc + dc[q] + 2) >> 1) - 1;
+      const bool in = (unsigned)(r + dr[q]) < (unsigned)th && (unsigned)(c + dc[q]) < (unsigned)tw;
+      const float* x = (qc < COLOUR ? xn : xo) + qc * nq;
+      v[q] = in ? x[qi + (size_t)rh * qj] : 0.0f;
+      t[q] = __ldg(cf + (size_t)q * 4 * nq + k);
+    }
+    const float L = __ldg(cf + (size_t)8 * 4 * nq + k);
     float s = 0.0f;
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-      const int qq = (q[j] >= 0 && q[j] < b.np) ? q[j] : 0;  // absent neighbours: index 1 in the reference
-      const float t = x[qq] * cf[1 + j];
-      s = j == 0 ? t : s + t;
+    for (int q = 0; q < 8; q++) {
+      const float a = v[q] * t[q];
+      s = q == 0 ? a : s + a;
     }
-    x[p] = cf[9] - s;
+    xn[(size_t)COLOUR * nq + k] = L - s;
   }
 }
 
-// Energy partial sums of the frames due for a check: sum over masked p of x_p (Q x)_p (FP64) and
-// of Le_p x_p (FP32), kRcParts CTAs per frame over fixed pixel ranges.
-__global__ void __launch_bounds__(256) k_rc_energy(RcBufs b, int nf, const int* __restrict__ due, double regfac,
-                                                   double vf2) {
+// Linear energy terms of iterates it0 .. it0 + nit - 1 (slots sl.x ..) of the frames that have swept that
+// far: FP32 sums of Le_p x_p, kRcParts CTAs per frame over fixed pixel ranges.
+__global__ void __launch_bounds__(256) k_rc_linear(RcBufs b, int it0, int nit, int4 sl, const int* __restrict__ limit) {
   const int f = blockIdx.y;
-  if (!due[f]) return;
+  if (limit[f] < it0 + nit - 1) return;
   const int th = b.th, np = b.np;
-  const double* ww = b.ww + (size_t)f * np * kRcStencil;
-  const uint8_t* mk = b.mask + (size_t)f * np;
-  const float* x = b.x + (size_t)f * np;
   const float* le = b.le + (size_t)f * np;
+  const float* xs[kRcBatch] = {rc_iterate(b, sl.x, f), rc_iterate(b, sl.y, f), rc_iterate(b, sl.z, f),
+                               rc_iterate(b, sl.w, f)};
   const int per = (np + kRcParts - 1) / kRcParts, a = blockIdx.x * per, e = min(np, a + per);
-  double qs = 0.0;
-  float ls = 0.0f;
+  float ls[kRcBatch] = {};
   for (int p = a + threadIdx.x; p < e; p += blockDim.x) {
-    if (!mk[p]) continue;
-    const double xp = (double)x[p];
-    double qx = rc_q(b, ww, mk, p, p, regfac, vf2) * xp;
-    const int nb[8] = {p - 1, p + 1, p - th + 1, p + th - 1, p - th, p + th, p - th - 1, p + th + 1};
+    const int c = p / th, r = p - c * th;
+    const size_t at = rc_place(b, r, c);
+    const float l = le[p];  // zero at unmasked pixels
 #pragma unroll
-    for (int j = 0; j < 8; j++)
-      if (nb[j] >= 0 && nb[j] < np) qx += rc_q(b, ww, mk, p, nb[j], regfac, vf2) * (double)x[nb[j]];
-    qs += xp * qx;
-    ls += le[p] * x[p];
+    for (int k = 0; k < kRcBatch; k++)
+      if (k < nit) ls[k] = fmaf(l, xs[k][at], ls[k]);
   }
-  __shared__ double sq[256];
-  __shared__ float sl[256];
-  sq[threadIdx.x] = qs;
-  sl[threadIdx.x] = ls;
+  __shared__ float sv[kRcBatch][256];
+#pragma unroll
+  for (int k = 0; k < kRcBatch; k++) sv[k][threadIdx.x] = ls[k];
   __syncthreads();
   for (int o = 128; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-      sq[threadIdx.x] += sq[threadIdx.x + o];
-      sl[threadIdx.x] += sl[threadIdx.x + o];
-    }
+    if (threadIdx.x < o)
+#pragma unroll
+      for (int k = 0; k < kRcBatch; k++) sv[k][threadIdx.x] += sv[k][threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    b.part[((size_t)f * kRcParts + blockIdx.x)] = sq[0];
-    b.part_l[(size_t)f * kRcParts + blockIdx.x] = sl[0];
+  if (threadIdx.x < nit) b.part_l[((size_t)f * kRcBatch + threadIdx.x) * kRcParts + blockIdx.x] = sv[threadIdx.x][0];
+}
+
+// Quadratic energy terms of those iterates: FP64 sums of x_p (Q x)_p over masked p, each pair of pixels
+// once. A thread takes a 2 x 2 quad, the same place of the four quarter planes, so that consecutive
+// lanes read consecutive floats of an iterate, a quad's 11 samples are converted once each, and its 20
+// stencil entries (five times an iterate's bytes) serve nit iterates: 376 us for four iterates of 64
+// frames of 512 x 512, with the linear terms 506; one iterate at a time took 4 x 125 with a thread and
+// 20 conversions per pixel. kRcParts CTAs per frame.
+__global__ void __launch_bounds__(256) k_rc_quadratic(RcBufs b, int it0, int nit, int4 sl, const int* __restrict__ limit,
+                                                      double regfac, double vf2) {
+  const int f = blockIdx.y;
+  if (limit[f] < it0 + nit - 1) return;
+  const int th = b.th, tw = b.tw, np = b.np, rh = b.rh;
+  const size_t nq = b.nq;
+  const double* ww = b.ww + (size_t)f * np * kRcStencil;
+  const uint8_t* mk = b.mask + (size_t)f * np;
+  const int s_ne = th == 2 ? 1 : 2;  // (offset th - 1 is S there)
+  double qs[kRcBatch] = {};
+  for (int k = blockIdx.x * 256 + threadIdx.x; k < b.nq; k += kRcParts * 256) {
+    const int j = k / rh, i = k - j * rh, r0 = 2 * i, c0 = 2 * j;
+    auto masked = [&](int r, int c) {
+      return (unsigned)r < (unsigned)th && (unsigned)c < (unsigned)tw && mk[(size_t)c * th + r] != 0;
+    };
+    // masks of the quad and its neighbours: rows r0 - 1 .. r0 + 2, columns c0 .. c0 + 2
+    bool m[4][3];
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+      for (int e = 0; e < 3; e++) m[a][e] = masked(r0 - 1 + a, c0 + e);
+    // Q(p, q) of the quad's pixels (r0 + dr, c0 + dc) with themselves and their S, NE, E, SE neighbours
+    double q[2][2][kRcStencil];
+#pragma unroll
+    for (int dr = 0; dr < 2; dr++)
+#pragma unroll
+      for (int dc = 0; dc < 2; dc++) {
+        double* v = q[dr][dc];
+        const int r = r0 + dr, c = c0 + dc;
+#pragma unroll
+        for (int s = 0; s < kRcStencil; s++) v[s] = 0.0;
+        if (!m[1 + dr][dc]) continue;
+        const size_t p = (size_t)c * th + r;
+        const int nh = (c > 0) + (c < tw - 1), nv = (r > 0) + (r < th - 1);
+        v[0] = ww[p] + regfac * ((double)nh + (double)nv * vf2);
+        if (m[2 + dr][dc]) v[1] = ww[(size_t)np + p] - regfac * vf2;
+        if (th == 2) v[1] += v[1];  // (p + 1 and p + th - 1 are both summed there)
+        if (m[dr][dc + 1]) v[2] = ww[(size_t)s_ne * np + p];
+        if (m[1 + dr][dc + 1]) v[3] = ww[(size_t)3 * np + p] - regfac;
+        if (m[2 + dr][dc + 1]) v[4] = ww[(size_t)4 * np + p];
+      }
+    const bool up = r0 > 0, down = r0 + 2 < th, low = r0 + 1 < th, right = c0 + 2 < tw, mid = c0 + 1 < tw;
+#pragma unroll
+    for (int t = 0; t < kRcBatch; t++) {
+      if (t >= nit) break;
+      const float* x = rc_iterate(b, t == 0 ? sl.x : t == 1 ? sl.y : t == 2 ? sl.z : sl.w, f) + k;
+      const float *A = x, *B = x + nq, *C = x + 2 * nq, *D = x + 3 * nq;
+      // rows r0 - 1 .. r0 + 2, columns c0 .. c0 + 2
+      const double a0 = A[0], b0 = mid ? B[0] : 0.f, c_0 = low ? C[0] : 0.f, d0 = low && mid ? D[0] : 0.f;
+      const double a_r = right ? A[rh] : 0.f, c_r = right && low ? C[rh] : 0.f;
+      const double a_d = down ? A[1] : 0.f, b_d = down && mid ? B[1] : 0.f, a_dr = down && right ? A[rh + 1] : 0.f;
+      const double d_u = up && mid ? D[-1] : 0.f, c_ur = up && right ? C[rh - 1] : 0.f;
+      auto px = [](const double (&v)[kRcStencil], double p, double s, double ne, double e, double se) {
+        return p * (v[0] * p + 2.0 * (v[1] * s + v[2] * ne + v[3] * e + v[4] * se));
+      };
+      qs[t] += (px(q[0][0], a0, c_0, d_u, b0, d0) + px(q[0][1], b0, d0, c_ur, a_r, c_r)) +
+               (px(q[1][0], c_0, a_d, b0, d0, b_d) + px(q[1][1], d0, b_d, a_r, c_r, a_dr));
+    }
+  }
+  __shared__ double sq[kRcBatch][8];
+#pragma unroll
+  for (int t = 0; t < kRcBatch; t++) {
+    const double v = warp_sum(qs[t]);
+    if ((threadIdx.x & 31) == 0) sq[t][threadIdx.x >> 5] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x < nit) {
+    double v = 0.0;
+    for (int w = 0; w < 8; w++) v += sq[threadIdx.x][w];
+    b.part[((size_t)f * kRcBatch + threadIdx.x) * kRcParts + blockIdx.x] = v;
   }
 }
 
-// The check of every due frame (a thread per frame): the energy from its partial sums in a fixed
-// order; a frame whose energy did not decrease stops, else its iterate becomes the output candidate
-// (copied by k_rc_keep). eo[f] starts as the energy of the first iterate (check number 0).
-__global__ void k_rc_check(int nf, const int* __restrict__ due, int* __restrict__ state, float* __restrict__ eo,
-                           int* __restrict__ keep, const double* __restrict__ part, const float* __restrict__ part_l,
-                           int first, int it, int* __restrict__ iters) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= nf) return;
-  keep[f] = 0;
-  if (!due[f]) return;
+// The energies of those iterates (a thread each) from their partial sums in a fixed order.
+__global__ void k_rc_total(RcBufs b, int nf, int it0, int nit, const int* __restrict__ limit, float* __restrict__ energy) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x, f = e / kRcBatch, k = e - f * kRcBatch;
+  if (f >= nf || k >= nit || limit[f] < it0 + nit - 1) return;
   double q = 0.0;
   float l = 0.0f;
   for (int i = 0; i < kRcParts; i++) {
-    q += part[(size_t)f * kRcParts + i];
-    l += part_l[(size_t)f * kRcParts + i];
+    q += b.part[(size_t)e * kRcParts + i];
+    l += b.part_l[(size_t)e * kRcParts + i];
   }
-  const float e = (float)(q - 2.0 * (double)l);
-  if (first) {
-    eo[f] = e;
-    return;
-  }
-  if (eo[f] <= e) {
-    state[f] = 2;  // stopped
-    iters[f] = it;
-  } else {
-    eo[f] = e;
-    keep[f] = 1;
-  }
-}
-
-// Frames due for a check after sweep `it`: running, and `it` a multiple of their interval.
-__global__ void k_rc_due(int nf, const int* __restrict__ state, const int* __restrict__ interval, int it,
-                         int* __restrict__ due) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f < nf) due[f] = state[f] == 1 && it % interval[f] == 0;
+  energy[e] = (float)(q - 2.0 * (double)l);
 }
 
 // Masked pixels of every frame (a frame with none is skipped, as the reference's `continue`); grid
@@ -339,22 +418,17 @@ __global__ void __launch_bounds__(256) k_rc_count(RcBufs b, int* __restrict__ co
   }
 }
 
-// The candidate iterate of the frames whose check kept the sweep: xo = x; grid (blocks, frames).
-__global__ void __launch_bounds__(256) k_rc_keep(RcBufs b, const int* __restrict__ keep) {
-  const int f = blockIdx.y;
-  if (!keep[f]) return;
-  const size_t o = (size_t)f * b.np;
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < b.np; p += gridDim.x * blockDim.x) b.xo[o + p] = b.x[o + p];
-}
-
-// Output of a finished frame: its candidate iterate, NaN outside the mask.
+// Outputs of the chunk's frames: the iterate in slot[f] (below 0: zeros), NaN outside the mask.
 template <class OutT>
 __global__ void __launch_bounds__(256) k_rc_out(RcBufs b, int nf, OutT* __restrict__ out, uint8_t* __restrict__ mk_out,
-                                                const int* __restrict__ skip) {
+                                                const int* __restrict__ slot, const int* __restrict__ skip) {
   const size_t total = (size_t)b.np * nf;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-    const bool m = b.mask[e] && !skip[e / b.np];
-    out[e] = m ? (OutT)b.xo[e] : (OutT)NAN;
+    const int f = (int)(e / b.np), p = (int)(e - (size_t)f * b.np);
+    const bool m = b.mask[e] && !skip[f];
+    float v = 0.0f;
+    if (m && slot[f] >= 0) v = rc_iterate(b, slot[f], f)[rc_place(b, p % b.th, p / b.th)];
+    out[e] = m ? (OutT)v : (OutT)NAN;
     if (mk_out) mk_out[e] = m ? 1 : 0;
   }
 }

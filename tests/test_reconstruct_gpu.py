@@ -105,3 +105,26 @@ def test_frames_that_constrain_nothing_are_skipped():
     assert o_its[1] == 0
     m = o_mask
     np.testing.assert_allclose(g["data_corrected"][m], o_out[m], rtol=0, atol=1e-4 * np.abs(o_out[m]).max())
+
+
+def test_a_long_set_follows_the_interval_chain():
+    """More frames than one chunk (64) with different sweep counts and a skipped frame: the counts obey
+    the rule with the interval each frame's predecessor gave (multiples of it), and the iterates are
+    the oracle's at those sweeps."""
+    rec, s, dxk, dyk = _estimated(7, n_frames=12)
+    reps = 6  # 72 frames
+    fr = np.concatenate([rec.frames * (0.2 + 0.7 * k) for k in range(reps)], axis=2).astype(np.float32)
+    dxk, dyk = np.tile(dxk, (1, reps)), np.tile(dyk, (1, reps))
+    dxk = dxk + 0.13 * np.sin(np.arange(dxk.shape[1]))[None, :]
+    dxk[:, 65] += 1000.0
+    g = api.reconstruct_frames(fr, dxk, dyk, s, rec.template.shape)
+    its, n = list(g["iterations"]), 1
+    for it in its:
+        assert it % n == 0
+        if it:
+            n = int(max(1, min(10, rc.round_half_away(np.sqrt(np.float32(it))))))
+    assert its[65] == 0 and len(set(its)) > 3
+    o_out, o_mask, _ = _oracle(fr, dxk, dyk, s, rec.template.shape, stop_at=its)
+    np.testing.assert_array_equal(g["mask"], o_mask)
+    np.testing.assert_allclose(g["data_corrected"][o_mask], o_out[o_mask], rtol=0,
+                               atol=1e-4 * np.abs(o_out[o_mask]).max())
