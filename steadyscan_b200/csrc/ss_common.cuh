@@ -123,7 +123,9 @@ struct GroupDesc {
   const uint8_t* base_mask;
   const int* min_points;    // W
   const void* image;        // Hb x fW column-major, engine frame type
-  const void* tquad;        // (Ht-1)(Wt-1) template quads, engine template type
+  const void* tquad;        // (Ht-1)(Wt-1) template quads, engine template type; FP64: Ht rows of Wt
+  const int* geo_shared;    // precision 'D': 1 when every block column has column 0's tfrac and basex, basey
+                            // repeats every 32 rows and no row is masked (bit for bit), else 0
   const void* gquad;        // gradient quads or nullptr when derived from the template
   const double* sum_image; // sum of the frame data over all Hb x fW entries
   // state
@@ -181,7 +183,7 @@ struct Quad {
 template <class Acc, class TplT>
 __device__ __forceinline__ void load_quad(const void* base, size_t i, Acc& t00, Acc& t01, Acc& t10, Acc& t11);
 
-template <>
+template <>  // (gradients; FP64 template values are read from rows)
 __device__ __forceinline__ void load_quad<double, double>(const void* base, size_t i, double& a, double& b,
                                                           double& c, double& d) {
   const double2* q = reinterpret_cast<const double2*>(base) + 2 * i;

@@ -65,6 +65,28 @@ __global__ void k_build_tquad(const double* __restrict__ T, int Ht, int Wt, TplT
   }
 }
 
+// FP64 template rows from the column-major template.
+__global__ void k_build_trows(const double* __restrict__ T, int Ht, int Wt, double* __restrict__ out) {
+  const size_t n = (size_t)Ht * Wt;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    out[i] = T[(i % Wt) * Ht + i / Wt];
+}
+
+// GroupDesc::geo_shared of Hb x W geometry tables, compared bit for bit (*flag starts as 1).
+__global__ void __launch_bounds__(256) k_geo_shared(const double* __restrict__ frac, const double* __restrict__ bx,
+                                                    const double* __restrict__ by, const uint8_t* __restrict__ mask,
+                                                    int Hb, int W, int* __restrict__ flag) {
+  const size_t n = (size_t)Hb * W;
+  bool same = true;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const size_t c = i / Hb, r = i - c * Hb;
+    same = same && __double_as_longlong(frac[i]) == __double_as_longlong(frac[r]) &&
+           __double_as_longlong(bx[i]) == __double_as_longlong(bx[r]) &&
+           __double_as_longlong(by[i]) == __double_as_longlong(by[c * Hb + (r & 31)]) && mask[i] != 0;
+  }
+  if (!same) *flag = 0;
+}
+
 // FP32 template rows of `pitch` floats (zero padding) from the column-major FP64 template, the
 // source of the shared-memory row windows of precision 'S'.
 __global__ void k_build_tplain(const double* __restrict__ T, int Ht, int Wt, int pitch, float* __restrict__ out) {
@@ -229,10 +251,6 @@ constexpr int kStageBytes = 96 * 1024;
 #define SS_EVAL_WIN_KB 72
 #endif
 constexpr int kWinBytes = SS_EVAL_WIN_KB * 1024;
-// Shared memory for the template rows of one line-search CTA (98 rows of a 512-pixel template;
-// with the kernel's static shared memory one 1024-thread CTA per SM).
-constexpr int kLsWinBytes = 196 * 1024;
-
 // Grid of an evaluation launch: the CTAs of `fn` resident on the device at once with `smem` bytes,
 // at most the batch's tiles (the CTAs take tiles from the launch's schedule until it is exhausted).
 template <class F>
@@ -256,7 +274,7 @@ static int resident_grid(F* fn, int threads, size_t smem, int max_tiles) {
 using EvalFn = cudaError_t (*)(int mode, int max_tiles, cudaStream_t s, const GroupDesc* gd, int* sched, int cap,
                                const GroupCtl* ctl, int max_hb, int win_bytes);
 using LsFn = cudaError_t (*)(int frames, cudaStream_t s, const GroupDesc* gd, const int* fg, GroupCtl* ctl,
-                             int win_bytes);
+                             int geo_rows);
 using SumFn = void (*)(const void* img, size_t n, double* parts, double* out, cudaStream_t s);
 
 template <class Acc, class FrameT, class TplT>
@@ -286,20 +304,17 @@ static cudaError_t eval_launch(int mode, int max_tiles, cudaStream_t s, const Gr
   return cudaGetLastError();
 }
 
-template <class Acc, class FrameT, class TplT>
+// The cluster line search of precision 'D'; geo_rows: rows of shared geometry its CTAs have room for.
+template <class FrameT>
 static cudaError_t ls_launch(int frames, cudaStream_t s, const GroupDesc* gd, const int* fg, GroupCtl* ctl,
-                             int win_bytes) {
-  if (sizeof(Acc) != 4) win_bytes = 0;
-  win_bytes = std::min(win_bytes, kLsWinBytes) & ~15;
-  if (win_bytes) {
-    cudaError_t ae = smem_attr(k_linesearch<Acc, FrameT, TplT>, kLsWinBytes + 16);
-    if (ae != cudaSuccess) return ae;
-  }
+                             int geo_rows) {
+  cudaError_t ae = smem_attr(k_linesearch<FrameT>, kLsGeoBytes);
+  if (ae != cudaSuccess) return ae;
   if (frames <= 0) return cudaSuccess;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(frames * kLsCluster, 1, 1);
-  cfg.blockDim = dim3(LsShape<Acc>::threads, 1, 1);
-  cfg.dynamicSmemBytes = win_bytes ? (size_t)win_bytes + 16 : 0;
+  cfg.blockDim = dim3(kLsThreads, 1, 1);
+  cfg.dynamicSmemBytes = (size_t)geo_rows * 2 * sizeof(double);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -308,7 +323,7 @@ static cudaError_t ls_launch(int frames, cudaStream_t s, const GroupDesc* gd, co
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_linesearch<Acc, FrameT, TplT>, gd, fg, ctl, win_bytes);
+  return cudaLaunchKernelEx(&cfg, k_linesearch<FrameT>, gd, fg, ctl, geo_rows);
 }
 
 using RoundFn = cudaError_t (*)(int max_tiles, cudaStream_t s, const GroupDesc* gd, int* tsched, int n_frames,
@@ -350,7 +365,7 @@ static cudaError_t sched_launch(int mode, cudaStream_t s, const GroupDesc* gd, c
 
 struct KernelSet {
   EvalFn eval;
-  LsFn ls;
+  LsFn ls;        // precision 'D' only
   RoundFn round;  // precision 'S' only
 };
 template <class FrameT>
@@ -362,9 +377,9 @@ static void sum_launch(const void* img, size_t n, double* parts, double* out, cu
 template <class Acc, class FrameT, class TplT>
 static KernelSet kset() {
   if constexpr (sizeof(Acc) == 4)
-    return {eval_launch<Acc, FrameT, TplT>, ls_launch<Acc, FrameT, TplT>, round_launch<FrameT, TplT>};
+    return {eval_launch<Acc, FrameT, TplT>, nullptr, round_launch<FrameT, TplT>};
   else
-    return {eval_launch<Acc, FrameT, TplT>, ls_launch<Acc, FrameT, TplT>, nullptr};
+    return {eval_launch<Acc, FrameT, TplT>, ls_launch<FrameT>, nullptr};
 }
 
 static KernelSet pick_kernels(int compute, int fdt, int tdt) {
@@ -779,7 +794,7 @@ struct Batch::Impl {
   double* d_sum_parts = nullptr;            // partial sums of k_sum_image
   unsigned long long h_staging[kStagingCounters] = {};
   int win_bytes = 0;          // template window bytes per assembly/final CTA (0: no windows)
-  int ls_win_bytes = 0;       // template window bytes per line-search CTA (0: no windows)
+  int ls_geo_rows = 0;        // rows of shared geometry of a line-search CTA (precision 'D')
   int* h_counters = nullptr;  // pinned
   int n_tiles = 0, n_chunks = 0, n_frames_total = 0;
   int n_trial_tiles = 0;  // most tiles a trial round can have
@@ -855,7 +870,7 @@ struct Batch::Impl {
     }
     if (mode == kTrial && ks.round)
       ks.round(n_trial_tiles, stream, d_gd, d_tsched, n_frames_total, (int)gd.size(), d_ctl, win_bytes);
-    else if (mode == kTrial) ks.ls(n_frames_total, stream, d_gd, d_frame_group, d_ctl, ls_win_bytes);
+    else if (mode == kTrial) ks.ls(n_frames_total, stream, d_gd, d_frame_group, d_ctl, ls_geo_rows);
     else ks.eval(mode, n_tiles, stream, d_gd, d_sched, n_chunks, d_ctl, max_hb, win_bytes);
     if (timing) {
       cudaEventRecord(events[event_used + 1], stream);
@@ -915,7 +930,7 @@ static void layout(Batch::Impl* b, char* base) {
   b->d_sum_parts = cv.take<double>(kSumBlocks);
   if (!b->early) b->d_ready = b->stream_req ? cv.take<int>(std::max<size_t>(1, b->hg.size())) : nullptr;
   b->win_bytes = 0;
-  b->ls_win_bytes = 0;
+  b->ls_geo_rows = 0;
   for (size_t i = 0; i < b->hg.size(); i++) {
     HostGroup& g = b->hg[i];
     GroupDesc& G = gd[i];
@@ -930,6 +945,8 @@ static void layout(Batch::Impl* b, char* base) {
     b->n_tiles += g.W * ((g.nF + g.frames_per_cta - 1) / g.frames_per_cta);
     b->n_trial_tiles += g.W * ((g.nF + kTrialTileFrames - 1) / kTrialTileFrames);
     b->n_chunks += (g.nF + g.frames_per_cta - 1) / g.frames_per_cta;
+    if (b->compute == 0 && (size_t)g.Hb * 2 * sizeof(double) <= (size_t)kLsGeoBytes)
+      b->ls_geo_rows = std::max(b->ls_geo_rows, g.Hb);
     if (!(b->compute == 1 && g.geo_k > 0)) b->max_hb = std::max(b->max_hb, g.Hb);  // affine: no tables
     G.frame_base = b->n_frames_total;
     b->n_frames_total += g.nF;
@@ -947,6 +964,7 @@ static void layout(Batch::Impl* b, char* base) {
       G.frac = S.frac; G.basex = S.basex; G.basey = S.basey;
       G.frac_f = S.frac_f; G.basex_f = S.basex_f; G.basey_f = S.basey_f;
       G.base_mask = S.base_mask; G.min_points = S.min_points;
+      G.geo_shared = S.geo_shared;
       G.col_yrange = S.col_yrange;
     } else {
       G.frac = cv.take<double>(hbw);
@@ -961,6 +979,7 @@ static void layout(Batch::Impl* b, char* base) {
       }
       G.base_mask = cv.take<uint8_t>(hbw);
       G.min_points = cv.take<int>(g.W);
+      G.geo_shared = b->compute == 0 ? cv.take<int>(1) : nullptr;
       G.col_yrange = b->compute == 1 ? cv.take<float>(2 * (size_t)g.W) : nullptr;
     }
     G.err = b->d_err;
@@ -983,7 +1002,7 @@ static void layout(Batch::Impl* b, char* base) {
       G.tplain = S.tplain;
       G.tpitch = S.tpitch;
     } else {
-      G.tquad = cv.take<char>(nq * 4 * tsz);
+      G.tquad = cv.take<char>(b->tpl_dt == SS_F64 ? (size_t)g.Ht * g.Wt * tsz : nq * 4 * tsz);
       G.gquad = g.grad_derived ? nullptr : cv.take<char>(nq * 4 * tsz);
       // precision 'S' with an FP32 template and derived gradients samples row windows in shared
       // memory: rows padded to 16 bytes for the bulk copies
@@ -1307,6 +1326,10 @@ int Batch::prepare(int n, const ss_inputs* in, ss_outputs* out, void* external, 
       }
       SS_CK(stg.put((void*)G.base_mask, g.bmask.data(), hbw));
       SS_CK(stg.put((void*)G.min_points, g.minp.data(), g.W * 4));
+      if (G.geo_shared) {
+        k_set_flag<<<1, 1, 0, s>>>((int*)G.geo_shared);
+        k_geo_shared<<<148, 256, 0, s>>>(G.frac, G.basex, G.basey, G.base_mask, g.Hb, g.W, (int*)G.geo_shared);
+      }
       if (G.col_yrange) {  // [min, max] of basey over the valid rows of each block column
         const double* BY = g.by.data();
         g.yrange.assign(2 * (size_t)g.W, 0.0f);
@@ -1349,7 +1372,7 @@ int Batch::prepare(int n, const ss_inputs* in, ss_outputs* out, void* external, 
     if (g.tpl_src != -1) {
       // template quads shared with an earlier group or held by a session
     } else if (b->tpl_dt == SS_F64) {
-      k_build_tquad<double><<<nb, 256, 0, s>>>(g.d_templ_stage, g.Ht, g.Wt, (double*)G.tquad);
+      k_build_trows<<<nb, 256, 0, s>>>(g.d_templ_stage, g.Ht, g.Wt, (double*)G.tquad);
       if (!g.grad_derived)
         k_build_gquad<double><<<nb, 256, 0, s>>>(g.d_xg_stage, g.d_yg_stage, g.Ht, g.Wt, (double*)G.gquad);
     } else if (b->tpl_dt == SS_F32) {
@@ -1600,7 +1623,7 @@ static int prime_attributes(Batch::Impl* b) {
   if (b->ks.round)
     SS_CK(b->ks.round(0, b->stream, b->d_gd, b->d_tsched, b->n_frames_total, (int)b->gd.size(), b->d_ctl,
                       b->win_bytes));
-  else SS_CK(b->ks.ls(0, b->stream, b->d_gd, b->d_frame_group, b->d_ctl, b->ls_win_bytes));
+  else SS_CK(b->ks.ls(0, b->stream, b->d_gd, b->d_frame_group, b->d_ctl, b->ls_geo_rows));
   return SS_OK;
 }
 
@@ -1650,7 +1673,7 @@ static int build_run_graph(Batch::Impl* b) {
       b->ks.eval(kCorr, b->n_tiles, s, b->d_gd, sc, nc, b->d_ctl, b->max_hb, b->win_bytes);
     }
   } else {
-    b->ks.ls(b->n_frames_total, s, b->d_gd, b->d_frame_group, b->d_ctl, b->ls_win_bytes);
+    b->ks.ls(b->n_frames_total, s, b->d_gd, b->d_frame_group, b->d_ctl, b->ls_geo_rows);
   }
   k_after_ls<<<nG, kAfterLsThreads, 0, s>>>(b->d_gd, b->d_ctl);
   k_iter_sums<<<dim3(kIterSplit, nG), 256, 0, s>>>(b->d_gd, b->d_ctl);
@@ -1914,7 +1937,7 @@ struct Server::Impl {
   bool configured = false;
   int compute = 0, frame_dt = 0, tpl_dt = 0;
   KernelSet ks = {nullptr, nullptr, nullptr};
-  int max_hb = 0, win_bytes = 0, ls_win_bytes = 0;
+  int max_hb = 0, win_bytes = 0, ls_geo_rows = 0;
   std::vector<Slot> slots;
   std::vector<GroupDesc> h_gd;
   GroupCtl* h_ctl = nullptr;  // pinned: the slots' control state after each cycle
@@ -2031,7 +2054,7 @@ int Server::admit(const ss_inputs* in, ss_outputs* out, const Batch* session, vo
   }
   v->max_hb = std::max(v->max_hb, bi->max_hb);
   v->win_bytes = std::max(v->win_bytes, bi->win_bytes);
-  v->ls_win_bytes = std::max(v->ls_win_bytes, bi->ls_win_bytes);
+  v->ls_geo_rows = std::max(v->ls_geo_rows, bi->ls_geo_rows);
   Impl::Slot& sl = v->slots[slot];
   sl.batch = b;
   sl.joining = true;
@@ -2135,7 +2158,7 @@ int Server::step() {
     sched_launch(kCorr, s, v->d_gd, v->d_ctl, v->d_chunk_group, nc, sc);
     v->ks.eval(kCorr, v->n_tiles, s, v->d_gd, sc, nc, v->d_ctl, v->max_hb, v->win_bytes);
   } else {
-    v->ks.ls(v->n_frames, s, v->d_gd, v->d_frame_group, v->d_ctl, v->ls_win_bytes);
+    v->ks.ls(v->n_frames, s, v->d_gd, v->d_frame_group, v->d_ctl, v->ls_geo_rows);
   }
   k_after_ls<<<nG, kAfterLsThreads, 0, s>>>(v->d_gd, v->d_ctl);
   k_iter_sums<<<dim3(kIterSplit, nG), 256, 0, s>>>(v->d_gd, v->d_ctl);

@@ -68,16 +68,13 @@ struct MinBlocks<float, MODE> {
 constexpr int kTrialMinBlocks = SS_TRIAL_MIN_BLOCKS;
 constexpr int kTrialWinBytes = SS_TRIAL_WIN_KB * 1024;
 
-// Line-search CTA: 256 threads; two (FP64) or four (FP32) CTAs per SM. A launch given window bytes
-// keeps the template rows of the CTA's knot range in shared memory for the whole search.
-template <class Acc>
-struct LsShape {
-  static constexpr int threads = 256, min_blocks = 2;
-};
-template <>
-struct LsShape<float> {
-  static constexpr int threads = 256, min_blocks = 4;
-};
+// Line-search CTA (FP64). A block column's tfrac and basex are staged in shared memory for the whole
+// search where all columns share them (GroupDesc::geo_shared) and they fit.
+#ifndef SS_LS_BLOCKS
+#define SS_LS_BLOCKS 3
+#endif
+constexpr int kLsThreads = 256;
+constexpr int kLsGeoBytes = 64 * 1024;
 
 __device__ __forceinline__ bool frame_active(const GroupDesc& G, int f, int shift) {
   // groupActive[groupId + shift * nGroups] with zero-filled reads past the array
@@ -154,9 +151,11 @@ __device__ __forceinline__ bool warp_pixel(Acc kx0, Acc kx1, Acc ky0, Acc ky1, A
 
 // Integer part and fraction of a non-negative coordinate, as static_cast<int> in the reference.
 __device__ __forceinline__ int split(double x, double& frac) {
-  int i = (int)x;
-  frac = x - (double)i;
-  return i;
+  // x + 2^52 rounded down holds floor(x) in its mantissa (0 <= x < 2^31): additions in place of two
+  // conversions at a quarter of the FP64 rate
+  const double v = __dadd_rd(x, 4503599627370496.0);
+  frac = x - (v - 4503599627370496.0);
+  return __double2loint(v);
 }
 __device__ __forceinline__ int split(float x, float& frac) {
   // x + 2^23 rounded down holds floor(x) in its mantissa (0 <= x < 2^23)
@@ -171,7 +170,8 @@ struct Sample {
 };
 
 // Bilinear template value and warped gradients at a valid pixel (task_differenceimage.cuh:118-126,
-// task_updategradients.cu:12-20). With gquad == nullptr the gradients are the template's forward
+// task_updategradients.cu:12-20). FP64 templates are rows, whose corners neighbouring lanes share in
+// L1; a 32-byte quad per pixel made the FP64 passes L2-bound. With gquad == nullptr the gradients are the template's forward
 // differences (steady_scan.m:178-179), taken from the same four template values.
 template <class Acc, class TplT, bool kGrad>
 __device__ __forceinline__ Sample<Acc> sample(const GroupDesc& G, Acc x, Acc y) {
@@ -179,7 +179,15 @@ __device__ __forceinline__ Sample<Acc> sample(const GroupDesc& G, Acc x, Acc y) 
   const int ix = split(x, xf), iy = split(y, yf);
   const size_t qi = (size_t)iy * (size_t)(G.Wt - 1) + (size_t)ix;
   Acc t00, t01, t10, t11;
-  load_quad<Acc, TplT>(G.tquad, qi, t00, t01, t10, t11);
+  if constexpr (sizeof(TplT) == 8) {
+    const double* q = reinterpret_cast<const double*>(G.tquad) + (size_t)iy * G.Wt + ix;
+    t00 = __ldg(q);
+    t01 = __ldg(q + 1);
+    t10 = __ldg(q + G.Wt);
+    t11 = __ldg(q + G.Wt + 1);
+  } else {
+    load_quad<Acc, TplT>(G.tquad, qi, t00, t01, t10, t11);
+  }
   const Acc one = (Acc)1;
   Acc a = fma(yf, t10, (one - yf) * t00);
   Acc b = fma(yf, t11, (one - yf) * t01);
@@ -226,6 +234,14 @@ template <class Acc, class FrameT>
 __device__ __forceinline__ Acc ld_pixel(const void* base, size_t i) {
   return (Acc)to_double(ld_frame<FrameT>(base, i));
 }
+__device__ __forceinline__ double pixel_double(uint16_t v) {  // 2^52 + v has v in its mantissa
+  return __hiloint2double(0x43300000, v) - 4503599627370496.0;
+}
+__device__ __forceinline__ double pixel_double(__half v) { return to_double(v); }
+template <>
+__device__ __forceinline__ double ld_pixel<double, uint16_t>(const void* base, size_t i) {
+  return pixel_double(ld_frame<uint16_t>(base, i));
+}
 template <>
 __device__ __forceinline__ float ld_pixel<float, uint16_t>(const void* base, size_t i) {
   return (float)ld_frame<uint16_t>(base, i);
@@ -260,8 +276,9 @@ struct ColGeo {
   const Acc* frac;
   const Acc* bx;
   const Acc* by;
-  const uint8_t* bm;
-  const Acc* fnext;  // tfrac of column (c+1) mod W; equals frac when all columns match
+  const uint8_t* bm;  // null: every row valid
+  const Acc* fnext;   // tfrac of column (c+1) mod W; equals frac when all columns match
+  int by_rows = -1;   // row r's basey is by[r & by_rows]
 };
 
 template <class Acc>
@@ -326,8 +343,8 @@ __device__ __forceinline__ void eval_column(const GroupDesc& G, size_t coli, con
     } else if (in) {
       f = geo.frac[r];
       bxv = geo.bx[r];
-      byv = geo.by[r];
-      bm = geo.bm[r] != 0;
+      byv = geo.by[r & geo.by_rows];
+      bm = geo.bm == nullptr || geo.bm[r] != 0;
     }
     Acc x, y;
     const bool mA = warp_pixel<Acc>(k.ax0, k.ax1, k.ay0, k.ay1, f, bxv, byv, bm, tw, th, x, y) && in;
@@ -426,70 +443,233 @@ __device__ __forceinline__ void eval_column(const GroupDesc& G, size_t coli, con
   for (int i = 0; i < NS; i++) out[i] = warp_sum((double)s[i]);
 }
 
-// Trial SSD and valid count of up to NC block columns of one frame with one warp, their rows
-// interleaved so that the frame loads and template gathers of all columns are in flight together.
-// Loads are predicated by index clamping (a masked pixel reads row 0 / quad 0 and is discarded), so
-// the column loop has no divergent branches. tq: frame-local column indices, nq <= NC of them valid.
-template <class Acc, class FrameT, class TplT, bool AFFINE, int NC, bool WIN = false>
-__device__ __forceinline__ void trial_columns(const GroupDesc& G, int b0, const TWin& win, const int (&tq)[NC], int nq,
-                                              const Acc (&qx0)[NC], const Acc (&qx1)[NC], const Acc (&qy0)[NC],
-                                              const Acc (&qy1)[NC], double (&ssd)[NC], int (&cnt)[NC]) {
-  const int lane = threadIdx.x & 31;
-  const int Hb = G.Hb;
-  const Acc tw = Limits<Acc>::lim(G.Wt), th = Limits<Acc>::lim(G.Ht);
-  Acc s[NC];
-  int c[NC];
-  size_t coli[NC];
-  ColGeo<Acc> geo[NC];
-  Acc aby[NC];
-  Acc a_j = 0, a_dj = 0, a_f0 = 0;
-  if (AFFINE) {
-    const int l = lane % G.geo_k;
-    a_j = (Acc)(lane / G.geo_k);
-    a_dj = (Acc)(32 / G.geo_k);
-    a_f0 = ((Acc)(l * G.geo_L) + (Acc)0.5) * (Acc)G.geo_fs;
+// FP64 columns: the rows of a warp's step and the loads of one lane's. RUN 1: kStep row steps of 32
+// consecutive rows; RUN 4: each lane takes 4 consecutive rows, as vector loads. Rows are pixel by pixel,
+// k lines each, so with 4 or more lines per knot lanes 4 rows apart sample neighbouring template columns
+// of one line, and a gather touches 2 or 3 cache lines in place of 4 to 8 (k = 4, 512 pixels: 120 -> 62
+// L1 wavefronts per 128 rows).
+constexpr int kStep = 4;
+template <int RUN>
+__device__ __forceinline__ int step_row(int q) {
+  return RUN == 4 ? 4 * (threadIdx.x & 31) + q : 32 * q + (threadIdx.x & 31);
+}
+template <int RUN>
+__device__ __forceinline__ void step_doubles(const double* p, int r0, int rb, double (&v)[kStep]) {
+  if constexpr (RUN == 4) {  // (rb is a multiple of 4)
+    const int r = r0 + step_row<4>(0);
+    const double2* q = reinterpret_cast<const double2*>(p + (r < rb ? r : 0));
+    const double2 a = q[0], b = q[1];
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+  } else {
 #pragma unroll
-    for (int q = 0; q < NC; q++) aby[q] = fma((Acc)G.geo_ay, (Acc)(tq[q] * G.geo_k + l), (Acc)G.geo_by);
-  }
-#pragma unroll
-  for (int q = 0; q < NC; q++) {
-    s[q] = (Acc)0;
-    c[q] = 0;
-    coli[q] = (size_t)(b0 + tq[q]) * Hb;
-    if (!AFFINE) geo[q] = global_geo<Acc>(G, tq[q]);
-  }
-  for (int r0 = 0; r0 < Hb; r0 += 32) {
-    const int r = r0 + lane;
-    const bool in = r < Hb;
-    const int rr = in ? r : 0;
-    Acc fa = 0, bxa = 0;
-    if (AFFINE) {
-      fa = fma((Acc)G.geo_fs, a_j, a_f0);
-      bxa = fma((Acc)G.geo_ax, a_j, (Acc)G.geo_bx);
-      a_j += a_dj;
+    for (int q = 0; q < kStep; q++) {
+      const int r = r0 + step_row<1>(q);
+      v[q] = p[r < rb ? r : 0];
     }
+  }
+}
+template <int RUN, class FrameT>
+__device__ __forceinline__ void step_frame(const void* img, size_t coli, int r0, int rb, double (&v)[kStep]) {
+  if constexpr (RUN == 4) {
+    const int r = r0 + step_row<4>(0);
+    const FrameT* p = reinterpret_cast<const FrameT*>(img) + coli + (r < rb ? r : 0);
+    if constexpr (sizeof(FrameT) == 8) {
+      const double2 a = __ldg(reinterpret_cast<const double2*>(p)), b = __ldg(reinterpret_cast<const double2*>(p) + 1);
+      v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+    } else if constexpr (sizeof(FrameT) == 4) {
+      const float4 a = __ldg(reinterpret_cast<const float4*>(p));
+      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    } else {
+      const uint2 a = __ldg(reinterpret_cast<const uint2*>(p));
+      const FrameT* e = reinterpret_cast<const FrameT*>(&a);
 #pragma unroll
-    for (int q = 0; q < NC; q++) {
-      if (q < nq) {
-        const Acc f = AFFINE ? fa : geo[q].frac[rr];
-        const Acc bx = AFFINE ? bxa : geo[q].bx[rr];
-        const Acc by = AFFINE ? aby[q] : geo[q].by[rr];
-        const bool bm = AFFINE ? in : (in && geo[q].bm[rr] != 0);
-        Acc x, y;
-        const bool m = warp_pixel<Acc>(qx0[q], qx1[q], qy0[q], qy1[q], f, bx, by, bm, tw, th, x, y);
-        const Acc img = ld_pixel<Acc, FrameT>(G.image, coli[q] + rr);
-        const Acc wI = samp<Acc, TplT, false, WIN>(G, win, m ? x : (Acc)0, m ? y : (Acc)0).wI;
-        const Acc d = img - wI;
-        s[q] = m ? fma(d, d, s[q]) : s[q];
-        c[q] += m ? 1 : 0;
+      for (int q = 0; q < kStep; q++) v[q] = pixel_double(e[q]);
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < kStep; q++) {
+      const int r = r0 + step_row<1>(q);
+      v[q] = ld_pixel<double, FrameT>(img, coli + (r < rb ? r : 0));
+    }
+  }
+}
+// The frame's columns may be read by 4-row vectors (runs of 4 rows aligned to 4 samples).
+template <class FrameT>
+__device__ __forceinline__ bool run4_ok(const GroupDesc& G) {
+  constexpr int kAlign = sizeof(FrameT) >= 4 ? 16 : 8;
+  return G.Hb % 4 == 0 && reinterpret_cast<uintptr_t>(G.image) % kAlign == 0 && G.Hb >= 4 &&
+         G.basex[0] == G.basex[1] && G.basex[0] == G.basex[2] && G.basex[0] == G.basex[3];
+}
+
+// Trial SSD and valid count of one block column with one warp (FP64). The kStep rows of a lane's step
+// are evaluated together, their frame loads and template gathers in flight at once; loads
+// are predicated by index clamping (a masked pixel reads row 0 / pixel (0, 0) and is discarded).
+template <class FrameT, int RUN>
+__device__ __forceinline__ void trial_column(const GroupDesc& G, size_t coli, const ColGeo<double>& geo, double kx0,
+                                             double kx1, double ky0, double ky1, double& ssd, int& cnt) {
+  const int rb = G.Hb;
+  const double tw = Limits<double>::lim(G.Wt), th = Limits<double>::lim(G.Ht);
+  double s = 0.0;
+  int c = 0;
+#pragma unroll 1
+  for (int r0 = 0; r0 < rb; r0 += 32 * kStep) {
+    double img[kStep], x[kStep], y[kStep], fr[kStep], bx[kStep];
+    bool m[kStep];
+    step_frame<RUN, FrameT>(G.image, coli, r0, rb, img);
+    step_doubles<RUN>(geo.frac, r0, rb, fr);
+    step_doubles<RUN>(geo.bx, r0, rb, bx);
+#pragma unroll
+    for (int q = 0; q < kStep; q++) {
+      const int r = r0 + step_row<RUN>(q), rr = r < rb ? r : 0;
+      const bool bm = r < rb && (geo.bm == nullptr || geo.bm[rr] != 0);
+      m[q] = warp_pixel<double>(kx0, kx1, ky0, ky1, fr[q], bx[q], geo.by[rr & geo.by_rows], bm, tw, th, x[q], y[q]);
+    }
+    double wI[kStep];
+#pragma unroll
+    for (int q = 0; q < kStep; q++) wI[q] = sample<double, double, false>(G, m[q] ? x[q] : 0.0, m[q] ? y[q] : 0.0).wI;
+#pragma unroll
+    for (int q = 0; q < kStep; q++) {
+      const double d = img[q] - wI[q];
+      s = m[q] ? fma(d, d, s) : s;
+      c += m[q] ? 1 : 0;
+    }
+  }
+  ssd = warp_sum(s);
+  cnt = warp_sum(c);
+}
+
+// Assembly sums of one block column with one warp (FP64), the mask and difference-image knots the same
+// and every block column's tfrac the same: eval_column<kAssemble>'s arithmetic, two rows of a lane's step
+// at a time (the recording above: 4.8 -> 3.3 ms of assembly a run). Its SSD adds in trial_column's order: a trial that moves no knot gives the same sum.
+template <class FrameT, int RUN>
+__device__ __forceinline__ void assemble_column(const GroupDesc& G, size_t coli, const ColGeo<double>& geo,
+                                                const ColKnots<double>& k, double (&out)[kCsStride], int& cnt_out) {
+  const int Hb = G.Hb;
+  const double tw = Limits<double>::lim(G.Wt), th = Limits<double>::lim(G.Ht);
+  double s[kCsAssemble] = {};
+  int cnt = 0;
+#pragma unroll 1
+  for (int r0 = 0; r0 < Hb; r0 += 32 * kStep) {
+    double img[kStep], fr[kStep], bx[kStep];
+    step_frame<RUN, FrameT>(G.image, coli, r0, Hb, img);
+    step_doubles<RUN>(geo.frac, r0, Hb, fr);
+    step_doubles<RUN>(geo.bx, r0, Hb, bx);
+#pragma unroll
+    for (int h = 0; h < kStep; h += 2) {
+      Sample<double> sa[2];
+      bool m[2];
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int r = r0 + step_row<RUN>(h + e), rr = r < Hb ? r : 0;
+        const bool bm = r < Hb && (geo.bm == nullptr || geo.bm[rr] != 0);
+        double x, y;
+        m[e] = warp_pixel<double>(k.ax0, k.ax1, k.ay0, k.ay1, fr[h + e], bx[h + e], geo.by[rr & geo.by_rows], bm, tw, th,
+                                  x, y);
+        sa[e] = sample<double, double, true>(G, m[e] ? x : 0.0, m[e] ? y : 0.0);
+      }
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        cnt += m[e] ? 1 : 0;
+        const double f = fr[h + e];
+        const double wx = m[e] ? sa[e].wx : 0.0, wy = m[e] ? sa[e].wy : 0.0, d = m[e] ? img[h + e] - sa[e].wI : 0.0;
+        const double fsq = f * f, csq = (1.0 - f) * (1.0 - f), fc = f - fsq;
+        const double gxx = wx * wx, gyy = wy * wy, gxy = wx * wy;
+        s[kCsSsd] = fma(d, d, s[kCsSsd]);
+        s[kCsAxx] = fma(gxx, csq, s[kCsAxx]);
+        s[kCsAyy] = fma(gyy, csq, s[kCsAyy]);
+        s[kCsAxy] = fma(gxy, csq, s[kCsAxy]);
+        s[kCsBxx] = fma(gxx, fsq, s[kCsBxx]);
+        s[kCsByy] = fma(gyy, fsq, s[kCsByy]);
+        s[kCsBxy] = fma(gxy, fsq, s[kCsBxy]);
+        s[kCsOxx] = fma(gxx, fc, s[kCsOxx]);
+        s[kCsOyy] = fma(gyy, fc, s[kCsOyy]);
+        s[kCsOxy] = fma(gxy, fc, s[kCsOxy]);
+        const double d1 = d * (1.0 - f), d2 = d * f;
+        s[kCsJ1x] = fma(d1, wx, s[kCsJ1x]);
+        s[kCsJ1y] = fma(d1, wy, s[kCsJ1y]);
+        s[kCsJ2x] = fma(d2, wx, s[kCsJ2x]);
+        s[kCsJ2y] = fma(d2, wy, s[kCsJ2y]);
       }
     }
   }
+  cnt_out = warp_sum(cnt);
 #pragma unroll
-  for (int q = 0; q < NC; q++) {
-    ssd[q] = warp_sum((double)s[q]);
-    cnt[q] = warp_sum(c[q]);
+  for (int i = 0; i < kCsAssemble; i++) out[i] = warp_sum(s[i]);
+}
+
+// Correlation sums (kCsSumD .. kCsFrDI; MODE kFinal also kCsFinalSsd and the mask output) of
+// one block column with one warp (FP64), the mask and difference-image knots the same:
+// eval_column<kCorr / kFinal>'s arithmetic without DiffState. The leading run of valid pixels follows the
+// row order, which with RUN 4 is lane by lane.
+template <class FrameT, int MODE, int RUN>
+__device__ __forceinline__ void corr_column(const GroupDesc& G, size_t coli, const ColGeo<double>& geo,
+                                            const ColKnots<double>& k, double (&out)[kCsStride], int& cnt_out,
+                                            uint8_t* mask_out) {
+  const int rb = G.Hb, lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const double tw = Limits<double>::lim(G.Wt), th = Limits<double>::lim(G.Ht);
+  constexpr int NS = nsums(MODE);
+  double s[NS] = {};
+  int cnt = 0;
+  bool run = true;
+#pragma unroll 1
+  for (int r0 = 0; r0 < rb; r0 += 32 * kStep) {
+    double img[kStep], fr[kStep], bx[kStep], wA[kStep];
+    bool m[kStep], pre[kStep];
+    step_frame<RUN, FrameT>(G.image, coli, r0, rb, img);
+    step_doubles<RUN>(geo.frac, r0, rb, fr);
+    step_doubles<RUN>(geo.bx, r0, rb, bx);
+#pragma unroll
+    for (int q = 0; q < kStep; q++) {
+      const int r = r0 + step_row<RUN>(q), rr = r < rb ? r : 0;
+      const bool bm = r < rb && (geo.bm == nullptr || geo.bm[rr] != 0);
+      double x, y;
+      m[q] = warp_pixel<double>(k.ax0, k.ax1, k.ay0, k.ay1, fr[q], bx[q], geo.by[rr & geo.by_rows], bm, tw, th, x, y);
+      wA[q] = sample<double, double, false>(G, m[q] ? x : 0.0, m[q] ? y : 0.0).wI;
+      if (MODE == kFinal && mask_out && r < rb) mask_out[r] = m[q] ? 1 : 0;
+    }
+    // pixels of the leading run: all pixels before them in row order are valid, and they are
+    if constexpr (RUN == 4) {
+      const unsigned bal = __ballot_sync(0xffffffffu, m[0] && m[1] && m[2] && m[3]);
+      bool p = run && (bal & lt) == lt;
+#pragma unroll
+      for (int q = 0; q < kStep; q++) pre[q] = p = p && m[q];
+      run = run && bal == 0xffffffffu;
+    } else {
+#pragma unroll
+      for (int q = 0; q < kStep; q++) {
+        const unsigned bal = __ballot_sync(0xffffffffu, m[q]);
+        pre[q] = run && m[q] && (bal & lt) == lt;
+        run = run && bal == 0xffffffffu;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kStep; q++) {
+      cnt += m[q] ? 1 : 0;
+      const double v = img[q], dA = v - wA[q], dp = m[q] ? v - dA : 0.0;  // dp: after d_swapWIDiff
+      s[kCsSumD] += dp;
+      const double vs = pre[q] ? v : 0.0, ds = pre[q] ? dp : 0.0;
+      s[kCsSetN] += pre[q] ? 1.0 : 0.0;
+      s[kCsSetD] += ds;
+      s[kCsSetDD] = fma(ds, ds, s[kCsSetDD]);
+      s[kCsSetI] += vs;
+      s[kCsSetII] = fma(vs, vs, s[kCsSetII]);
+      s[kCsSetDI] = fma(ds, vs, s[kCsSetDI]);
+      const double vm = m[q] ? v : 0.0;
+      s[kCsFrD] += dp;
+      s[kCsFrI] += vm;
+      s[kCsFrDD] = fma(dp, dp, s[kCsFrDD]);
+      s[kCsFrII] = fma(vm, vm, s[kCsFrII]);
+      s[kCsFrDI] = fma(dp, vm, s[kCsFrDI]);
+      if (MODE == kFinal) {
+        const double e = m[q] ? dA : 0.0;
+        s[kCsFinalSsd] = fma(e, e, s[kCsFinalSsd]);
+      }
+    }
   }
+  cnt_out = warp_sum(cnt);
+#pragma unroll
+  for (int i = 0; i < NS; i++) out[i] = warp_sum(s[i]);
 }
 
 // Shared-memory bytes of one staged block column of geometry (tfrac, basex, basey, the next
@@ -627,6 +807,7 @@ __device__ __forceinline__ void eval_tile(const GroupDesc& G, const GroupCtl& C,
     atomicAdd(G.staging + 0, 1ull);
     if (win.p) atomicAdd(G.staging + 1, 1ull);
   }
+  const bool run4 = sizeof(Acc) == 8 && run4_ok<FrameT>(G);
   for (int f = fb * fpc + warp; f < f_end; f += kEvalWarps) {
     const int c = f * W + cc;
     ColKnots<Acc> k;
@@ -676,6 +857,16 @@ __device__ __forceinline__ void eval_tile(const GroupDesc& G, const GroupCtl& C,
         if (affine) eval_column<Acc, FrameT, TplT, MODE, true>(G, coli, geo, k, out, cnt, mo, cc);
         else eval_column<Acc, FrameT, TplT, MODE>(G, coli, geo, k, out, cnt, mo);
       }
+    } else if (MODE == kAssemble && G.frac_uniform && !k.dual) {
+      if constexpr (sizeof(Acc) == 8) {
+        if (run4) assemble_column<FrameT, 4>(G, coli, geo, k, out, cnt);
+        else assemble_column<FrameT, 1>(G, coli, geo, k, out, cnt);
+      }
+    } else if (MODE != kAssemble && !k.dual) {
+      if constexpr (sizeof(Acc) == 8) {
+        if (run4) corr_column<FrameT, MODE, 4>(G, coli, geo, k, out, cnt, mo);
+        else corr_column<FrameT, MODE, 1>(G, coli, geo, k, out, cnt, mo);
+      }
     } else {
       eval_column<Acc, FrameT, TplT, MODE>(G, coli, geo, k, out, cnt, mo);
     }
@@ -717,18 +908,23 @@ __global__ void __launch_bounds__(32 * kEvalWarps, MinBlocks<Acc, MODE>::value)
 }
 
 // Line search of one frame per thread-block cluster (task_linesearch.cu:76-149), for every frame of
-// every group in kPhHalf. The cluster's CTAs split the frame's block columns; each trial's SSD,
-// valid count, block presence and largest step are reduced across the cluster through distributed
-// shared memory, rank 0 decides, and every CTA applies the decision to its own copy of the knots, so
-// the frame's whole search runs without leaving the kernel. The frame's right boundary knot is the
-// committed knot at line-search start (p_snap), or the never-written 1e6 for the last frame.
-// After shift 1 the cluster also evaluates the frame's correlation sums (the iteration-end state).
-template <class Acc, class FrameT, class TplT>
-__global__ void __launch_bounds__(LsShape<Acc>::threads, LsShape<Acc>::min_blocks)
+// every group in kPhHalf (precision 'D'; 'S' searches in trial rounds). The cluster's CTAs split the
+// frame's block columns; each trial's SSD, valid count, block presence and largest step are reduced
+// across the cluster through distributed shared memory, rank 0 decides, and every CTA applies the
+// decision to its own copy of the knots, so the frame's whole search runs without leaving the kernel.
+// The frame's right boundary knot is the committed knot at line-search start (p_snap), or the
+// never-written 1e6 for the last frame. After shift 1 the cluster also evaluates the frame's
+// correlation sums (the iteration-end state).
+// Bound: latency of the frame loads and template gathers (L1 wavefronts 45% of their peak, the FP64 pipe
+// 20%). 400 frames of 256 x 512 FP64, knots every 4 lines: 13.7 ms of searches a run with geometry tables
+// and template quads read per pixel (65 bytes from L2) and a row step at a time, 9.5 with template rows,
+// shared geometry and four steps in flight, 8.0 with runs of four rows, 7.0 with the correlation pass in
+// the same form and three CTAs per SM (two: 7.6; 16 warps a CTA and half the CTAs: 11.7).
+template <class FrameT>
+__global__ void __launch_bounds__(kLsThreads, SS_LS_BLOCKS)
     k_linesearch(const GroupDesc* __restrict__ gds, const int* __restrict__ frame_group, GroupCtl* __restrict__ ctl,
-                 int win_bytes) {
-  constexpr int kLsThreads = LsShape<Acc>::threads;
-  extern __shared__ __align__(16) unsigned char ls_smem[];
+                 int geo_rows) {
+  extern __shared__ __align__(16) double ls_geo[];  // tfrac, then basex, of geo_rows rows
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
   const int gf = blockIdx.x / kLsCluster;
@@ -771,51 +967,27 @@ __global__ void __launch_bounds__(LsShape<Acc>::threads, LsShape<Acc>::min_block
       s_kd[d][i] = G.kdiff[(size_t)f * 2 * (W + 1) + d * (W + 1) + t];
     }
   }
-  __syncthreads();
-
-  // Precision 'S': stage the template rows of this CTA's lines for every knot vector the search
-  // and the correlation pass can evaluate (trial knots lie between p and p + deltaP; kmask and
-  // kdiff are earlier states); a range that does not fit uses the global template.
-  TWin win{nullptr, 0, 0, 0};
-  uint64_t* stage_bar = nullptr;  // set when a staging copy timed out (drained before the CTA exits)
-  unsigned stage_phase = 0;
-  if constexpr (sizeof(Acc) == 4) {
-    const int win_cap = G.tplain ? win_bytes / (G.tpitch * (int)sizeof(float)) : 0;
-    if (win_cap >= 2 && !G.gquad && hi > lo) {
-      float klo = INFINITY, khi = -INFINITY;
-      for (int i = threadIdx.x; i < nk; i += blockDim.x) {
-        const float a = (float)s_p[1][i], b = (float)(s_p[1][i] + s_dp[1][i]);
-        const float c = (float)s_km[1][i], d = (float)s_kd[1][i];
-        klo = fminf(klo, fminf(fminf(a, b), fminf(c, d)));
-        khi = fmaxf(khi, fmaxf(fmaxf(a, b), fmaxf(c, d)));
-      }
-      float ylo = INFINITY, yhi = -INFINITY;
-      for (int t = lo + threadIdx.x; t < hi; t += blockDim.x) {
-        ylo = fminf(ylo, G.col_yrange[2 * t]);
-        yhi = fmaxf(yhi, G.col_yrange[2 * t + 1]);
-      }
-      block_minmax(klo, khi);
-      block_minmax(ylo, yhi);
-      int r0, rows;
-      window_rows(G, ylo + klo, yhi + khi, win_cap, r0, rows);
-      if (rows > 0) {
-        float* wbuf = reinterpret_cast<float*>(ls_smem);
-        uint64_t* bar = reinterpret_cast<uint64_t*>(ls_smem + (size_t)win_bytes);
-        if (threadIdx.x == 0) mbar_init(bar);
-        __syncthreads();
-        if (stage_window(G, wbuf, r0, rows, bar, stage_phase)) win = {wbuf, r0, rows, G.tpitch};
-        else stage_bar = bar;
-      }
+  const bool shared_geo = *G.geo_shared != 0, staged = shared_geo && Hb <= geo_rows;
+  if (staged)
+    for (int r = threadIdx.x; r < Hb; r += blockDim.x) {
+      ls_geo[r] = __ldg(G.frac + r);
+      ls_geo[Hb + r] = __ldg(G.basex + r);
     }
-  }
-  bool pairs = false;
-  if constexpr (sizeof(Acc) == 4) pairs = win.p && G.pair_ok;
-  if (threadIdx.x == 0) {
-    atomicAdd(G.staging + 2, 1ull);
-    if (win.p) atomicAdd(G.staging + 3, 1ull);
-    if (pairs) atomicAdd(G.staging + 4, 1ull);
-  }
-
+  __syncthreads();
+  auto column_geo = [&](int t) {
+    ColGeo<double> geo = global_geo<double>(G, t);
+    if (shared_geo) {
+      geo.by_rows = 31;
+      geo.bm = nullptr;
+    }
+    if (staged) {
+      geo.frac = geo.fnext = ls_geo;
+      geo.bx = ls_geo + Hb;
+    }
+    return geo;
+  };
+  if (threadIdx.x == 0) atomicAdd(G.staging + 2, 1ull);
+  const bool run4 = run4_ok<FrameT>(G);
   const double thr = G.move_thresh, rho = G.ls_mult;
   int trials = 0;
   while (searching) {
@@ -823,55 +995,19 @@ __global__ void __launch_bounds__(LsShape<Acc>::threads, LsShape<Acc>::min_block
     double ssd = 0, maxabs = 0, reg = 0;
     long long cnt = 0;
     bool present = false;
-    constexpr int NC = 4;
-    if (pairs) {
-      for (int t = lo + warp; t < hi; t += nw) {
-        const int i = t - lo;
-        const float x0 = (float)(s_p[0][i] + s_dp[0][i]), y0 = (float)(s_p[1][i] + s_dp[1][i]);
-        const float x1 = (float)((t + 1 < W) ? s_p[0][i + 1] + s_dp[0][i + 1] : s_p[0][i + 1]);
-        const float y1 = (float)((t + 1 < W) ? s_p[1][i + 1] + s_dp[1][i + 1] : s_p[1][i + 1]);
-        double qs;
-        int qc;
-        trial_pairs<FrameT>(G, (size_t)(b0 + t) * Hb, pair_col(G, t, x0, x1, y0, y1), pair_win(win), qs, qc);
-        ssd += qs;
-        cnt += qc;
-        present |= qc >= G.min_points[t];
-      }
-    }
-    for (int t0 = lo + warp; !pairs && t0 < hi; t0 += nw * NC) {
-      int tq[NC], nq = 0;
-      Acc qx0[NC], qx1[NC], qy0[NC], qy1[NC];
-#pragma unroll
-      for (int q = 0; q < NC; q++) {
-        int t = t0 + q * nw;
-        if (t >= hi) t = t0;  // padding column, not evaluated (nq excludes it)
-        else nq = q + 1;
-        const int i = t - lo;
-        tq[q] = t;
-        qx0[q] = (Acc)(s_p[0][i] + s_dp[0][i]);
-        qy0[q] = (Acc)(s_p[1][i] + s_dp[1][i]);
-        qx1[q] = (Acc)((t + 1 < W) ? s_p[0][i + 1] + s_dp[0][i + 1] : s_p[0][i + 1]);
-        qy1[q] = (Acc)((t + 1 < W) ? s_p[1][i + 1] + s_dp[1][i + 1] : s_p[1][i + 1]);
-      }
-      double qs[NC];
-      int qc[NC];
-      bool aff = false;
-      if constexpr (sizeof(Acc) == 4) aff = G.geo_k > 0;
-      if (win.p) {
-        if (aff) trial_columns<Acc, FrameT, TplT, true, NC, true>(G, b0, win, tq, nq, qx0, qx1, qy0, qy1, qs, qc);
-        else trial_columns<Acc, FrameT, TplT, false, NC, true>(G, b0, win, tq, nq, qx0, qx1, qy0, qy1, qs, qc);
-      } else {
-        if (aff) trial_columns<Acc, FrameT, TplT, true, NC>(G, b0, win, tq, nq, qx0, qx1, qy0, qy1, qs, qc);
-        else trial_columns<Acc, FrameT, TplT, false, NC>(G, b0, win, tq, nq, qx0, qx1, qy0, qy1, qs, qc);
-      }
-#pragma unroll
-      for (int q = 0; q < NC; q++) {
-        if (q < nq) {
-          ssd += qs[q];
-          cnt += qc[q];
-          present |= qc[q] >= G.min_points[tq[q]];
-        }
-      }
+    for (int t = lo + warp; t < hi; t += nw) {
+      const int i = t - lo;
+      const double x0 = s_p[0][i] + s_dp[0][i], y0 = s_p[1][i] + s_dp[1][i];
+      const double x1 = (t + 1 < W) ? s_p[0][i + 1] + s_dp[0][i + 1] : s_p[0][i + 1];
+      const double y1 = (t + 1 < W) ? s_p[1][i + 1] + s_dp[1][i + 1] : s_p[1][i + 1];
+      double qs;
+      int qc;
+      const size_t coli = (size_t)(b0 + t) * Hb;
+      if (run4) trial_column<FrameT, 4>(G, coli, column_geo(t), x0, x1, y0, y1, qs, qc);
+      else trial_column<FrameT, 1>(G, coli, column_geo(t), x0, x1, y0, y1, qs, qc);
+      ssd += qs;
+      cnt += qc;
+      present |= qc >= G.min_points[t];
     }
     for (int i = threadIdx.x; i < hi - lo; i += blockDim.x) {
       const int t = lo + i;
@@ -976,31 +1112,22 @@ __global__ void __launch_bounds__(LsShape<Acc>::threads, LsShape<Acc>::min_block
   if (shift == 1) {  // iteration-end correlation sums of this frame's state (task.cpp:284)
     for (int t = lo + warp; t < hi; t += nw) {
       const int i = t - lo;
-      ColKnots<Acc> k;
+      ColKnots<double> k;
       set_knots(k, s_km[0][i], s_km[0][i + 1], s_km[1][i], s_km[1][i + 1], s_kd[0][i], s_kd[0][i + 1], s_kd[1][i],
                 s_kd[1][i + 1]);
       double out[kCsStride];
       int c;
       const DiffState ds = diff_state<kCorr>(G, C.par_sel, shift, f, b0 + t);
-      if (ds.par_out || (G.flags & kFlagFrameCorr)) {  // the buffer state of flags M and c (DiffState)
-        eval_column<Acc, FrameT, TplT, kCorr, false, false, true>(G, (size_t)(b0 + t) * Hb, global_geo<Acc>(G, t), k,
-                                                                  out, c, nullptr, t, TWin{nullptr, 0, 0, 0}, ds);
-      } else if constexpr (sizeof(Acc) == 4) {
-        const size_t coli = (size_t)(b0 + t) * Hb;
-        if (win.p) {
-          if (G.geo_k > 0)
-            eval_column<Acc, FrameT, TplT, kCorr, true, true>(G, coli, global_geo<Acc>(G, t), k, out, c, nullptr, t, win);
-          else
-            eval_column<Acc, FrameT, TplT, kCorr, false, true>(G, coli, global_geo<Acc>(G, t), k, out, c, nullptr, t,
-                                                               win);
-        } else if (G.geo_k > 0) {
-          eval_column<Acc, FrameT, TplT, kCorr, true>(G, coli, global_geo<Acc>(G, t), k, out, c, nullptr, t);
-        } else {
-          eval_column<Acc, FrameT, TplT, kCorr>(G, coli, global_geo<Acc>(G, t), k, out, c, nullptr);
-        }
-      } else {
-        eval_column<Acc, FrameT, TplT, kCorr>(G, (size_t)(b0 + t) * Hb, global_geo<Acc>(G, t), k, out, c, nullptr);
-      }
+      const size_t coli = (size_t)(b0 + t) * Hb;
+      if (ds.par_out || (G.flags & kFlagFrameCorr))  // the buffer state of flags M and c (DiffState)
+        eval_column<double, FrameT, double, kCorr, false, false, true>(G, coli, column_geo(t), k, out, c, nullptr, t,
+                                                                       TWin{nullptr, 0, 0, 0}, ds);
+      else if (k.dual)
+        eval_column<double, FrameT, double, kCorr>(G, coli, column_geo(t), k, out, c, nullptr);
+      else if (run4)
+        corr_column<FrameT, kCorr, 4>(G, coli, column_geo(t), k, out, c, nullptr);
+      else
+        corr_column<FrameT, kCorr, 1>(G, coli, column_geo(t), k, out, c, nullptr);
       if (lane == 0) {
         double* dst = G.colsum + (size_t)(b0 + t) * kCsStride;
         for (int q = 0; q < nsums(kCorr); q++) dst[q] = out[q];
@@ -1008,7 +1135,6 @@ __global__ void __launch_bounds__(LsShape<Acc>::threads, LsShape<Acc>::min_block
       }
     }
   }
-  if (stage_bar) drain_window(stage_bar, stage_phase);  // uniform over the CTA
   cluster.sync();  // no CTA leaves while others may still read its shared memory
 }
 
