@@ -271,6 +271,22 @@ static int resident_grid(F* fn, int threads, size_t smem, int max_tiles) {
   return std::max(1, std::min(max_tiles, it->second));
 }
 
+// CTAs of a trial round resident on the device, over which its schedule spreads the tiles (ss_sched.cuh).
+static int trial_slots() {
+  static std::mutex mu;
+  static std::map<int, int> sms;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 148 * kTrialMinBlocks;
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = sms.find(dev);
+  if (it == sms.end()) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
+    it = sms.emplace(dev, n).first;
+  }
+  return it->second * kTrialMinBlocks;
+}
+
 using EvalFn = cudaError_t (*)(int mode, int max_tiles, cudaStream_t s, const GroupDesc* gd, int* sched, int cap,
                                const GroupCtl* ctl, int max_hb, int win_bytes);
 using LsFn = cudaError_t (*)(int frames, cudaStream_t s, const GroupDesc* gd, const int* fg, GroupCtl* ctl,
@@ -349,17 +365,16 @@ static cudaError_t round_launch(int max_tiles, cudaStream_t s, const GroupDesc* 
 // The trial schedule of the next round (one CTA).
 static cudaError_t trial_sched_launch(cudaStream_t s, const GroupDesc* gd, const GroupCtl* ctl, const int* frame_group,
                                       int n_frames, int n_groups, int* tsched) {
-  k_trial_schedule<<<1, kSchedThreads, 0, s>>>(gd, ctl, frame_group, n_frames, n_groups, tsched);
+  k_trial_schedule<<<1, kSchedThreads, 0, s>>>(gd, ctl, frame_group, n_frames, n_groups, tsched,
+                                               trial_slots());
   return cudaGetLastError();
 }
 
 // The schedule of an evaluation launch of `mode` (one CTA).
 static cudaError_t sched_launch(int mode, cudaStream_t s, const GroupDesc* gd, const GroupCtl* ctl,
                                 const int* chunk_group, int n_chunks, int* sched) {
-  if (mode == kAssemble) k_schedule<kAssemble><<<1, kSchedThreads, 0, s>>>(gd, ctl, chunk_group, n_chunks, sched, n_chunks);
-  else if (mode == kTrial) k_schedule<kTrial><<<1, kSchedThreads, 0, s>>>(gd, ctl, chunk_group, n_chunks, sched, n_chunks);
-  else if (mode == kCorr) k_schedule<kCorr><<<1, kSchedThreads, 0, s>>>(gd, ctl, chunk_group, n_chunks, sched, n_chunks);
-  else k_schedule<kFinal><<<1, kSchedThreads, 0, s>>>(gd, ctl, chunk_group, n_chunks, sched, n_chunks);
+  auto* fn = mode == kAssemble ? k_schedule<kAssemble> : mode == kCorr ? k_schedule<kCorr> : k_schedule<kFinal>;
+  fn<<<1, kSchedThreads, 0, s>>>(gd, ctl, chunk_group, n_chunks, sched, n_chunks);
   return cudaGetLastError();
 }
 
@@ -943,7 +958,7 @@ static void layout(Batch::Impl* b, char* base) {
     G.geo_ax = (float)g.geo_ax; G.geo_bx = (float)g.geo_bx; G.geo_ay = (float)g.geo_ay; G.geo_by = (float)g.geo_by;
     G.geo_fs = (float)g.geo_fs;
     b->n_tiles += g.W * ((g.nF + g.frames_per_cta - 1) / g.frames_per_cta);
-    b->n_trial_tiles += g.W * ((g.nF + kTrialTileFrames - 1) / kTrialTileFrames);
+    b->n_trial_tiles += g.W * ((g.nF + kTrialTileMin - 1) / kTrialTileMin);
     b->n_chunks += (g.nF + g.frames_per_cta - 1) / g.frames_per_cta;
     if (b->compute == 0 && (size_t)g.Hb * 2 * sizeof(double) <= (size_t)kLsGeoBytes)
       b->ls_geo_rows = std::max(b->ls_geo_rows, g.Hb);
@@ -1569,9 +1584,9 @@ __global__ void __launch_bounds__(kSchedThreads) k_sched_rounds(const GroupDesc*
                                                                 const GroupCtl* __restrict__ ctl,
                                                                 const int* __restrict__ frame_group, int n_frames,
                                                                 int n_groups, int* __restrict__ tsched,
-                                                                int* __restrict__ ctr, int first,
+                                                                int* __restrict__ ctr, int first, int slots,
                                                                 cudaGraphConditionalHandle h) {
-  const int tiles = build_trial_schedule(gds, ctl, frame_group, n_frames, n_groups, tsched);
+  const int tiles = build_trial_schedule(gds, ctl, frame_group, n_frames, n_groups, tsched, slots);
   if (threadIdx.x == 0) {
     if (first) ctr[kCtrRound] = 0;
     const bool more = tiles > 0 && ctr[kCtrRound] < kGraphRounds;
@@ -1666,7 +1681,7 @@ static int build_run_graph(Batch::Impl* b) {
   solve_launch(s, b->d_gd, b->d_ctl, nG);
   if (b->ks.round) {
     k_sched_rounds<<<1, kSchedThreads, 0, s>>>(b->d_gd, b->d_ctl, b->d_frame_group, b->n_frames_total, nG,
-                                               b->d_tsched, b->d_counters, 1, h_round);
+                                               b->d_tsched, b->d_counters, 1, trial_slots(), h_round);
     rc = capture_while(s, h_round, &rounds_body);
     if (!rc) {
       sched_launch(kCorr, s, b->d_gd, b->d_ctl, b->d_chunk_group, nc, sc);
@@ -1690,7 +1705,7 @@ static int build_run_graph(Batch::Impl* b) {
     SS_CK(cudaStreamBeginCaptureToGraph(s, rounds_body, nullptr, nullptr, 0, mode));
     b->ks.round(b->n_trial_tiles, s, b->d_gd, b->d_tsched, b->n_frames_total, nG, b->d_ctl, b->win_bytes);
     k_sched_rounds<<<1, kSchedThreads, 0, s>>>(b->d_gd, b->d_ctl, b->d_frame_group, b->n_frames_total, nG,
-                                               b->d_tsched, b->d_counters, 0, h_round);
+                                               b->d_tsched, b->d_counters, 0, trial_slots(), h_round);
     e = cudaStreamEndCapture(s, &out);
     if (e != cudaSuccess) return fail(SS_ERR_CUDA, std::string("run graph rounds: ") + cudaGetErrorString(e));
   }
@@ -2062,7 +2077,7 @@ int Server::admit(const ss_inputs* in, ss_outputs* out, const Batch* session, vo
   const HostGroup& g = bi->hg[0];
   sl.chunks = (g.nF + g.frames_per_cta - 1) / g.frames_per_cta;
   sl.tiles = g.W * sl.chunks;
-  sl.trial_tiles = g.W * ((g.nF + kTrialTileFrames - 1) / kTrialTileFrames);
+  sl.trial_tiles = g.W * ((g.nF + kTrialTileMin - 1) / kTrialTileMin);
   sl.frames = g.nF;
   GroupDesc G = bi->gd[0];
   G.err = v->d_err;

@@ -276,9 +276,9 @@ struct ColGeo {
   const Acc* frac;
   const Acc* bx;
   const Acc* by;
-  const uint8_t* bm;  // null: every row valid
+  const uint8_t* bm;  // FP64, null: every row valid
   const Acc* fnext;   // tfrac of column (c+1) mod W; equals frac when all columns match
-  int by_rows = -1;   // row r's basey is by[r & by_rows]
+  int by_rows = -1;   // FP64: row r's basey is by[r & by_rows]
 };
 
 template <class Acc>
@@ -343,8 +343,8 @@ __device__ __forceinline__ void eval_column(const GroupDesc& G, size_t coli, con
     } else if (in) {
       f = geo.frac[r];
       bxv = geo.bx[r];
-      byv = geo.by[r & geo.by_rows];
-      bm = geo.bm == nullptr || geo.bm[r] != 0;
+      byv = geo.by[sizeof(Acc) == 8 ? r & geo.by_rows : r];
+      bm = (sizeof(Acc) == 8 && geo.bm == nullptr) || geo.bm[r] != 0;
     }
     Acc x, y;
     const bool mA = warp_pixel<Acc>(k.ax0, k.ax1, k.ay0, k.ay1, f, bxv, byv, bm, tw, th, x, y) && in;
@@ -1168,6 +1168,7 @@ __device__ __forceinline__ int ld_acquire(const int* p) {
 }
 
 // Decision for frame f after all its columns of the round were evaluated (one warp).
+constexpr int kDecideBatch = 2;  // (4 spilled more in the trial loop: 46.1 ms of trial rounds against 44.6)
 __device__ __forceinline__ void ls_decide(const GroupDesc& G, GroupCtl& C, int f) {
   const int lane = threadIdx.x & 31;
   const int W = G.W, N = G.N, b0 = f * W, shift = C.shift;
@@ -1175,19 +1176,39 @@ __device__ __forceinline__ void ls_decide(const GroupDesc& G, GroupCtl& C, int f
   const double bx = G.p_snap[b0 + W], by = G.p_snap[N + b0 + W];
   double a = 0, m = 0, rg = 0, b = 0;
   bool pr = false;
-  for (int t = lane; t < W; t += 32) {
-    const int c = b0 + t;
-    a += __ldcg(G.colsum + (size_t)c * kCsStride + kCsSsd);
-    const int n = __ldcg(G.colcnt + c);
-    b += (double)n;
-    pr |= n >= G.min_points[t];
-    const double dx = G.delta_p[c], dy = G.delta_p[N + c];
-    m = fmax(m, fmax(fabs(dx), fabs(dy)));
+  // kDecideBatch knots of a lane loaded at once: the decision ends the round, and its loads one after
+  // the other were a third of a small round
+  for (int t0 = lane; t0 < W; t0 += 32 * kDecideBatch) {
+    double ss[kDecideBatch], dx[kDecideBatch], dy[kDecideBatch];
+    int n[kDecideBatch], mp[kDecideBatch];
+#pragma unroll
+    for (int q = 0; q < kDecideBatch; q++) {
+      const int t = t0 + 32 * q, c = b0 + t;
+      const bool in = t < W;
+      ss[q] = in ? __ldcg(G.colsum + (size_t)c * kCsStride + kCsSsd) : 0.0;
+      n[q] = in ? __ldcg(G.colcnt + c) : 0;
+      mp[q] = in ? G.min_points[t] : INT_MAX;
+      dx[q] = in ? G.delta_p[c] : 0.0;
+      dy[q] = in ? G.delta_p[N + c] : 0.0;
+    }
     if (G.lambda != 0.0) {  // knot-difference regulariser of the trial (extension)
-      const double x0 = G.p[c] + dx, y0 = G.p[N + c] + dy;
-      const double x1 = t + 1 < W ? G.p[c + 1] + G.delta_p[c + 1] : bx;
-      const double y1 = t + 1 < W ? G.p[N + c + 1] + G.delta_p[N + c + 1] : by;
-      rg += (x1 - x0) * (x1 - x0) + (y1 - y0) * (y1 - y0);
+#pragma unroll
+      for (int q = 0; q < kDecideBatch; q++) {
+        const int t = t0 + 32 * q, c = b0 + t;
+        if (t >= W) break;
+        const double x0 = G.p[c] + dx[q], y0 = G.p[N + c] + dy[q];
+        const double x1 = t + 1 < W ? G.p[c + 1] + G.delta_p[c + 1] : bx;
+        const double y1 = t + 1 < W ? G.p[N + c + 1] + G.delta_p[N + c + 1] : by;
+        rg += (x1 - x0) * (x1 - x0) + (y1 - y0) * (y1 - y0);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kDecideBatch; q++) {
+      if (t0 + 32 * q >= W) break;
+      a += ss[q];
+      b += (double)n[q];
+      pr |= n[q] >= mp[q];
+      m = fmax(m, fmax(fabs(dx[q]), fabs(dy[q])));
     }
   }
   a = warp_sum(a);
@@ -1223,16 +1244,32 @@ __device__ __forceinline__ void ls_decide(const GroupDesc& G, GroupCtl& C, int f
   const double rho = G.ls_mult;
   double* km = G.kmask + (size_t)f * 2 * (W + 1);
   double* kd = G.kdiff + (size_t)f * 2 * (W + 1);
-  for (int t = lane; t <= W; t += 32) {
-    for (int d = 0; d < 2; d++) {
-      const size_t o = (size_t)d * N + b0 + t;
-      const double v = t < W ? G.p[o] + G.delta_p[o] : (last_frame ? kPnewFill : (d ? by : bx));
-      km[d * (W + 1) + t] = v;
-      if (action & 16) kd[d * (W + 1) + t] = v;
-      if (t < W) {
-        if ((action & 15) == 0) G.p[o] = v;
-        else if ((action & 15) == 1) G.delta_p[o] *= rho;
-        else if (!(action & 16)) G.delta_p[o] *= rho;  // absent block: reduced before the stop test
+  const bool accept = (action & 15) == 0, shrink = (action & 15) == 1 || (!accept && !(action & 16));
+  for (int t0 = lane; t0 <= W; t0 += 32 * kDecideBatch) {
+    double p[kDecideBatch][2], dp[kDecideBatch][2];
+#pragma unroll
+    for (int q = 0; q < kDecideBatch; q++)
+#pragma unroll
+      for (int d = 0; d < 2; d++) {
+        const int t = t0 + 32 * q;
+        const size_t o = (size_t)d * N + b0 + t;
+        p[q][d] = t < W ? G.p[o] : 0.0;
+        dp[q][d] = t < W ? G.delta_p[o] : 0.0;
+      }
+#pragma unroll
+    for (int q = 0; q < kDecideBatch; q++) {
+      const int t = t0 + 32 * q;
+      if (t > W) break;
+#pragma unroll
+      for (int d = 0; d < 2; d++) {
+        const size_t o = (size_t)d * N + b0 + t;
+        const double v = t < W ? p[q][d] + dp[q][d] : (last_frame ? kPnewFill : (d ? by : bx));
+        km[d * (W + 1) + t] = v;
+        if (action & 16) kd[d * (W + 1) + t] = v;
+        if (t < W) {
+          if (accept) G.p[o] = v;
+          else if (shrink) G.delta_p[o] = dp[q][d] * rho;  // (an absent block: reduced before the stop test)
+        }
       }
     }
   }

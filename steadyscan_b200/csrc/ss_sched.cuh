@@ -129,27 +129,42 @@ __global__ void __launch_bounds__(kSchedThreads) k_schedule(const GroupDesc* __r
   build_schedule<MODE>(gds, ctl, chunk_group, n_chunks, sched, cap);
 }
 
+// Entry of a prefix list pre[0..n) that holds idx: the last one starting at or before it (one warp; the
+// result in every lane). Each turn narrows the range 32-fold by one load per lane, a round trip to
+// memory where a bisection takes five.
+__device__ __forceinline__ int find_entry(const int* __restrict__ pre, int n, int idx) {
+  const int lane = threadIdx.x & 31;
+  int lo = 0;
+  while (n > 1) {
+    const int step = (n + 31) >> 5, e = lo + lane * step;
+    const bool at = lane * step < n && pre[e] <= idx;
+    const int last = 31 - __clz(__ballot_sync(0xffffffffu, at) | 1u);
+    n = min(step, n - last * step);
+    lo += last * step;
+  }
+  return lo;
+}
+
 // The CTA's next tile of a scheduled launch into s_tile = (group, block column, frame chunk); false
 // (in every thread) when the list is exhausted. All threads call; s_tile is read until the caller's
 // next __syncthreads.
 __device__ __forceinline__ bool fetch_tile(int* __restrict__ sched, int cap, int* s_tile) {
-  if (threadIdx.x == 0) {
-    const int idx = atomicAdd(sched + kSchNext, 1);
-    if (idx >= sched[kSchTiles]) {
-      s_tile[0] = -1;
+  if (threadIdx.x < 32) {
+    int idx = threadIdx.x == 0 ? atomicAdd(sched + kSchNext, 1) : 0;
+    const int tiles = sched[kSchTiles], entries = sched[kSchEntries];
+    idx = __shfl_sync(0xffffffffu, idx, 0);
+    const int* grp = sched + kSchHdr;
+    const int* chk = grp + cap;
+    const int* pre = chk + cap;
+    if (idx >= tiles) {
+      if (threadIdx.x == 0) s_tile[0] = -1;
     } else {
-      const int* grp = sched + kSchHdr;
-      const int* chk = grp + cap;
-      const int* pre = chk + cap;
-      int lo = 0, hi = sched[kSchEntries] - 1;  // the last entry starting at or before idx
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (pre[mid] <= idx) lo = mid;
-        else hi = mid - 1;
+      const int e = find_entry(pre, entries, idx);
+      if (threadIdx.x == 0) {
+        s_tile[0] = grp[e];
+        s_tile[1] = idx - pre[e];
+        s_tile[2] = chk[e];
       }
-      s_tile[0] = grp[lo];
-      s_tile[1] = idx - pre[lo];
-      s_tile[2] = chk[lo];
     }
   }
   __syncthreads();
@@ -172,6 +187,10 @@ __device__ __forceinline__ bool fetch_tile(int* __restrict__ sched, int cap, int
 #define SS_TRIAL_TILE_FRAMES 32
 #endif
 constexpr int kTrialTileFrames = SS_TRIAL_TILE_FRAMES;
+constexpr int kTrialTileMin = 8;
+__device__ __forceinline__ int trial_tile_frames(long long columns, int slots) {
+  return columns >= 96LL * slots ? kTrialTileFrames : columns >= 32LL * slots ? 16 : kTrialTileMin;
+}
 
 // Buffer: header, list[nf] (batch frame index of each searching frame), first[ng] and end[ng] (each
 // group's run in the list), then grp[nf], pos[nf], cnt[nf] (entries) and prefix[nf + 1] (tiles).
@@ -219,7 +238,7 @@ __device__ __forceinline__ int cta_exclusive_scan(int v, int* total) {
 // its frame_base).
 __device__ __forceinline__ int build_trial_schedule(const GroupDesc* __restrict__ gds, const GroupCtl* __restrict__ ctl,
                                                     const int* __restrict__ frame_group, int n_frames, int n_groups,
-                                                    int* __restrict__ ts) {
+                                                    int* __restrict__ ts, int slots) {
   int* list = ts + kTsHdr;
   int* first = list + n_frames;
   int* end = first + n_groups;
@@ -228,7 +247,9 @@ __device__ __forceinline__ int build_trial_schedule(const GroupDesc* __restrict_
   int* cnt = pos + n_frames;
   int* pre = cnt + n_frames;
   __shared__ int s_base, s_base2, s_tiles;
+  __shared__ unsigned long long s_cols;  // block columns of the searching frames
   if (threadIdx.x == 0) {
+    s_cols = 0;
     s_base = 0;
     s_base2 = 0;
     s_tiles = 0;
@@ -248,20 +269,24 @@ __device__ __forceinline__ int build_trial_schedule(const GroupDesc* __restrict_
     int total;
     const int p = s_base + cta_exclusive_scan(s ? 1 : 0, &total);
     if (s) list[p] = j;
+    {
+      const int w = __reduce_add_sync(0xffffffffu, s ? gds[g].W : 0);
+      if ((threadIdx.x & 31) == 0 && w) atomicAdd(&s_cols, (unsigned long long)w);
+    }
     if (g >= 0 && f == 0) first[g] = p;
     if (g >= 0 && f == gds[g].nF - 1) end[g] = p + (s ? 1 : 0);
     if (threadIdx.x == 0) s_base += total;
     __syncthreads();
   }
-  const int n_list = s_base;
-  // entries: runs of up to kTrialTileFrames listed frames of one group
+  const int n_list = s_base, tile_frames = trial_tile_frames((long long)s_cols, slots);
+  // entries: runs of up to tile_frames listed frames of one group
   for (int p0 = 0; p0 < n_list; p0 += kSchedThreads) {
     const int p = p0 + threadIdx.x;
     int g = -1, w = 0;
     bool start = false;
     if (p < n_list) {
       g = frame_group[list[p]];
-      start = (p - first[g]) % kTrialTileFrames == 0;
+      start = (p - first[g]) % tile_frames == 0;
       w = start ? gds[g].W : 0;
     }
     int total_e, total_t;
@@ -270,7 +295,7 @@ __device__ __forceinline__ int build_trial_schedule(const GroupDesc* __restrict_
     if (start) {
       grp[e] = g;
       pos[e] = p;
-      cnt[e] = min(kTrialTileFrames, end[g] - p);
+      cnt[e] = min(tile_frames, end[g] - p);
       pre[e] = tp;
     }
     if (threadIdx.x == 0) {
@@ -291,32 +316,31 @@ __device__ __forceinline__ int build_trial_schedule(const GroupDesc* __restrict_
 __global__ void __launch_bounds__(kSchedThreads) k_trial_schedule(const GroupDesc* __restrict__ gds,
                                                                   const GroupCtl* __restrict__ ctl,
                                                                   const int* __restrict__ frame_group, int n_frames,
-                                                                  int n_groups, int* __restrict__ ts) {
-  build_trial_schedule(gds, ctl, frame_group, n_frames, n_groups, ts);
+                                                                  int n_groups, int* __restrict__ ts, int slots) {
+  build_trial_schedule(gds, ctl, frame_group, n_frames, n_groups, ts, slots);
 }
 
 // The CTA's next trial tile into s_tile = (group, block column, list position of its first frame,
 // frames); false (in every thread) when the list is exhausted. All threads call.
 __device__ __forceinline__ bool fetch_trial_tile(int* __restrict__ ts, int n_frames, int n_groups, int* s_tile) {
-  if (threadIdx.x == 0) {
-    const int idx = atomicAdd(ts + kTsNext, 1);
-    if (idx >= ts[kTsTiles]) {
-      s_tile[0] = -1;
+  if (threadIdx.x < 32) {
+    int idx = threadIdx.x == 0 ? atomicAdd(ts + kTsNext, 1) : 0;
+    const int tiles = ts[kTsTiles], entries = ts[kTsEntries];
+    idx = __shfl_sync(0xffffffffu, idx, 0);
+    const int* grp = ts + kTsHdr + n_frames + 2 * n_groups;
+    const int* pos = grp + n_frames;
+    const int* cnt = pos + n_frames;
+    const int* pre = cnt + n_frames;
+    if (idx >= tiles) {
+      if (threadIdx.x == 0) s_tile[0] = -1;
     } else {
-      const int* grp = ts + kTsHdr + n_frames + 2 * n_groups;
-      const int* pos = grp + n_frames;
-      const int* cnt = pos + n_frames;
-      const int* pre = cnt + n_frames;
-      int lo = 0, hi = ts[kTsEntries] - 1;  // the last entry starting at or before idx
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (pre[mid] <= idx) lo = mid;
-        else hi = mid - 1;
+      const int e = find_entry(pre, entries, idx);
+      if (threadIdx.x == 0) {
+        s_tile[0] = grp[e];
+        s_tile[1] = idx - pre[e];
+        s_tile[2] = pos[e];
+        s_tile[3] = cnt[e];
       }
-      s_tile[0] = grp[lo];
-      s_tile[1] = idx - pre[lo];
-      s_tile[2] = pos[lo];
-      s_tile[3] = cnt[lo];
     }
   }
   __syncthreads();
