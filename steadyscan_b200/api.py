@@ -152,7 +152,7 @@ def _result(o: SSOutputs, a: dict, dims) -> dict:
              frame_params=a["frame_params"].reshape(nF, 2 * (w + 1), order="F") if "frame_params" in a else None,
              blocks_used=a["blocks_used"].reshape(w, nF, order="F").astype(bool))
     if "mask" in a:
-        r["mask"] = a["mask"].reshape(hb, w * nF, order="F").astype(bool)
+        r["mask"] = a["mask"].view(np.bool_).reshape(hb, w * nF, order="F")  # 0 / 1 bytes
     r["rg_params"] = a["rg_params"].reshape(2 * N, 2 * mi, order="F") if "rg_params" in a else None
     r["function_times"] = a.get("function_times")
     r["iteration_times"] = a.get("iteration_times")
@@ -330,7 +330,7 @@ def reconstruct_frames(frames, dx_knots, dy_knots, settings: dict, template_shap
                       iters.ctypes.data, int(device))
     check(lib.ss_reconstruct_frames(C.byref(r)))
     del keep
-    return {"data_corrected": out, "mask": mask.astype(bool), "iterations": iters}
+    return {"data_corrected": out, "mask": mask.view(np.bool_), "iterations": iters}  # (the mask is 0 / 1 bytes)
 
 
 def recording_sets(n_frames: int, frames_per_set: int = 500, min_frames_per_set: int = 100):

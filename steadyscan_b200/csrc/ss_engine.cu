@@ -72,6 +72,39 @@ __global__ void k_build_trows(const double* __restrict__ T, int Ht, int Wt, doub
     out[i] = T[(i % Wt) * Ht + i / Wt];
 }
 
+// FP32 copies of the geometry tables (precision 'S').
+__global__ void __launch_bounds__(256) k_geo_single(const double* __restrict__ frac, const double* __restrict__ bx,
+                                                    const double* __restrict__ by, size_t n, float* __restrict__ f,
+                                                    float* __restrict__ x, float* __restrict__ y) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    f[i] = (float)frac[i];
+    x[i] = (float)bx[i];
+    y[i] = (float)by[i];
+  }
+}
+
+// [min, max] of basey over the valid rows of each block column (a warp per column).
+__global__ void __launch_bounds__(256) k_col_yrange(const double* __restrict__ by, const uint8_t* __restrict__ mask,
+                                                    int Hb, int W, float* __restrict__ range) {
+  const int c = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (c >= W) return;
+  double lo = INFINITY, hi = -INFINITY;
+  for (int r = lane; r < Hb; r += 32)
+    if (mask[(size_t)c * Hb + r]) {
+      const double v = by[(size_t)c * Hb + r];
+      lo = v < lo ? v : lo;
+      hi = hi < v ? v : hi;
+    }
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  if (lane == 0) {
+    range[2 * c] = (float)lo;
+    range[2 * c + 1] = (float)hi;
+  }
+}
+
 // GroupDesc::geo_shared of Hb x W geometry tables, compared bit for bit (*flag starts as 1).
 __global__ void __launch_bounds__(256) k_geo_shared(const double* __restrict__ frac, const double* __restrict__ bx,
                                                     const double* __restrict__ by, const uint8_t* __restrict__ mask,
@@ -222,6 +255,68 @@ static unsigned long long current_context_id() {
   if (get_current(&ctx) != CUDA_SUCCESS || !ctx) return 0;
   if (get_id(ctx, &id) != CUDA_SUCCESS) return 0;
   return id;
+}
+
+// Non-blocking streams kept for the next batch or call of the device (creating and destroying two or
+// three took 200 us of a small call). At most kPooledStreams wait; a stream comes back drained.
+constexpr size_t kPooledStreams = 16;
+struct PooledStream {
+  int dev;
+  unsigned long long ctx;
+  cudaStream_t s;
+};
+static std::mutex g_stream_mu;
+static std::vector<PooledStream> g_streams;
+
+static cudaError_t take_stream(cudaStream_t* out) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long ctx = current_context_id();
+  if (ctx) {
+    std::lock_guard<std::mutex> lock(g_stream_mu);
+    for (size_t i = 0; i < g_streams.size(); i++)
+      if (g_streams[i].dev == dev && g_streams[i].ctx == ctx) {
+        *out = g_streams[i].s;
+        g_streams.erase(g_streams.begin() + i);
+        return cudaSuccess;
+      }
+  }
+  return cudaStreamCreateWithFlags(out, cudaStreamNonBlocking);
+}
+
+// Gives a stream back (the caller has synchronised it); the device that it was taken on is current or
+// becomes so here.
+static void give_stream(cudaStream_t s, int dev) {
+  int cur = 0;
+  if (cudaGetDevice(&cur) == cudaSuccess && cur != dev) cudaSetDevice(dev);
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  const unsigned long long ctx = current_context_id();
+  const bool idle = cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone &&
+                    cudaStreamQuery(s) == cudaSuccess;
+  bool kept = false;
+  if (ctx && idle) {
+    std::lock_guard<std::mutex> lock(g_stream_mu);
+    // streams of a context that is gone are forgotten with it
+    g_streams.erase(std::remove_if(g_streams.begin(), g_streams.end(),
+                                   [&](const PooledStream& p) { return p.dev == dev && p.ctx != ctx; }),
+                    g_streams.end());
+    if (g_streams.size() < kPooledStreams) {
+      g_streams.push_back({dev, ctx, s});
+      kept = true;
+    }
+  }
+  if (!kept) cudaStreamDestroy(s);
+  if (cur != dev) cudaSetDevice(cur);
+}
+
+// Has the pages of a host output in place before its copy arrives (the bytes stay as they are): done
+// while the GPU works, since touching fresh pages costs as much as the copy.
+static void touch_pages(void* p, size_t n) {
+  if (!p || n < 65536) return;
+  volatile char* c = static_cast<volatile char*>(p);
+  for (size_t o = 0; o < n; o += 4096) c[o] = c[o];
+  c[n - 1] = c[n - 1];
 }
 
 // Opts a kernel into `bytes` of dynamic shared memory on the current device, once per device and
@@ -557,8 +652,6 @@ struct HostGroup {
   int frame_dt = SS_F64, tpl_dt = SS_F64;
   bool grad_derived = true, frac_uniform = true;
   HostDoubles templ, xg, yg, frac, bx, by, ex, ey;  // ex, ey: the initial knots
-  std::vector<float> frac_f, bx_f, by_f;  // precision 'S' geometry
-  std::vector<float> yrange;              // per block column [min, max] of basey over valid rows
   int frames_per_cta = 32;
   int tpl_src = -1, geo_src = -1;         // earlier group whose template / geometry buffers are shared,
                                           // or kFromSession
@@ -683,10 +776,16 @@ static int load_host_inputs(std::vector<HostGroup>& all, size_t gi) {
     if ((rc = host_doubles(in->tfrac, "tfrac", g.frac))) return rc;
     if ((rc = host_doubles(in->basex, "basex", g.bx))) return rc;
     if ((rc = host_doubles(in->basey, "basey", g.by))) return rc;
-    if ((rc = host_doubles(in->base_mask, "base_mask", tmp))) return rc;
-    g.bmask.resize(tmp.size());
-    const double* mk = tmp.data();
-    for (size_t i = 0; i < tmp.size(); i++) g.bmask[i] = mk[i] != 0.0;
+    if (in->base_mask.location == SS_HOST && in->base_mask.dtype == SS_U8 && in->base_mask.data) {
+      const uint8_t* mk = static_cast<const uint8_t*>(in->base_mask.data);
+      g.bmask.resize((size_t)g.Hb * g.W);
+      for (size_t i = 0; i < g.bmask.size(); i++) g.bmask[i] = mk[i] != 0;
+    } else {
+      if ((rc = host_doubles(in->base_mask, "base_mask", tmp))) return rc;
+      g.bmask.resize(tmp.size());
+      const double* mk = tmp.data();
+      for (size_t i = 0; i < tmp.size(); i++) g.bmask[i] = mk[i] != 0.0;
+    }
     if ((rc = host_doubles(in->min_points_per_block, "min_points_per_block", tmp))) return rc;
     g.minp.resize(g.W);
     const double* mp = tmp.data();
@@ -700,16 +799,19 @@ static int load_host_inputs(std::vector<HostGroup>& all, size_t gi) {
     const double* X = g.xg.data();
     const double* Y = g.yg.data();
     g.grad_derived = true;
-    for (int c = 0; c + 1 < g.Wt && g.grad_derived; c++)
-      for (int r = 0; r < g.Ht; r++) {
-        double d = T[(size_t)(c + 1) * g.Ht + r] - T[(size_t)c * g.Ht + r];
-        if (!(X[(size_t)c * g.Ht + r] == d)) { g.grad_derived = false; break; }
-      }
-    for (int c = 0; c < g.Wt && g.grad_derived; c++)
-      for (int r = 0; r + 1 < g.Ht; r++) {
-        double d = T[(size_t)c * g.Ht + r + 1] - T[(size_t)c * g.Ht + r];
-        if (!(Y[(size_t)c * g.Ht + r] == d)) { g.grad_derived = false; break; }
-      }
+    // (a column's differences without a branch per entry, so that the compiler vectorises the loops)
+    for (int c = 0; c + 1 < g.Wt && g.grad_derived; c++) {
+      const double *t = T + (size_t)c * g.Ht, *u = t + g.Ht, *x = X + (size_t)c * g.Ht;
+      long long bad = 0;
+      for (int r = 0; r < g.Ht; r++) bad += !(x[r] == u[r] - t[r]);
+      g.grad_derived = bad == 0;
+    }
+    for (int c = 0; c < g.Wt && g.grad_derived; c++) {
+      const double *t = T + (size_t)c * g.Ht, *y = Y + (size_t)c * g.Ht;
+      long long bad = 0;
+      for (int r = 0; r + 1 < g.Ht; r++) bad += !(y[r] == t[r + 1] - t[r]);
+      g.grad_derived = bad == 0;
+    }
   } else {
     g.grad_derived = g.tpl_src == kFromSession ? g.ses_hg->grad_derived : all[g.tpl_src].grad_derived;
   }
@@ -717,8 +819,7 @@ static int load_host_inputs(std::vector<HostGroup>& all, size_t gi) {
     g.frac_uniform = true;
     const double* F = g.frac.data();
     for (int c = 1; c < g.W && g.frac_uniform; c++)
-      for (int r = 0; r < g.Hb; r++)
-        if (std::memcmp(&F[(size_t)c * g.Hb + r], &F[r], sizeof(double)) != 0) { g.frac_uniform = false; break; }
+      g.frac_uniform = std::memcmp(F + (size_t)c * g.Hb, F, (size_t)g.Hb * sizeof(double)) == 0;
     if (g.compute == 1 && g.frac_uniform) detect_affine_geometry(g);
   } else {
     const HostGroup& s = g.geo_src == kFromSession ? *g.ses_hg : all[g.geo_src];
@@ -749,21 +850,22 @@ static void detect_affine_geometry(HostGroup& g) {
     const double by0 = BY[0];
     const double ay = (k > 1) ? BY[1] - BY[0] : (W > 1 ? BY[Hb] - BY[0] : 1.0);
     auto near = [](double a, double b) { return std::fabs(a - b) <= 1e-9 * std::max(1.0, std::fabs(b)); };
+    // block row r = j * k + l: pixel j of line cc * k + l. tfrac is the same in every column here (its
+    // first stands for all), basex usually is, and a line's basey usually one value: an entry equal to
+    // one already compared needs no comparison of its own.
     bool ok = true;
-    // block row r = j * k + l: pixel j of line cc * k + l
-    for (int cc = 0; cc < W && ok; cc++)
-      for (int j = 0; j < L && ok; j++) {
-        const double x = ax * j + bx0;
-        for (int l = 0; l < k; l++) {
-          const size_t i = (size_t)cc * Hb + (size_t)j * k + l;
-          const double f = ((double)l * L + j + 0.5) * fs;
-          const double y = ay * ((double)cc * k + l) + by0;
-          if (!MK[i] || !near(f, FR[i]) || !near(x, BX[i]) || !near(y, BY[i])) {
-            ok = false;
-            break;
-          }
-        }
-      }
+    for (int r = 0; r < Hb && ok; r++) ok = near(((double)(r % k) * L + r / k + 0.5) * fs, FR[r]);
+    for (int cc = 0; cc < W && ok; cc++) {
+      const double *X = BX + (size_t)cc * Hb, *Y = BY + (size_t)cc * Hb;
+      const uint8_t* M = MK + (size_t)cc * Hb;
+      long long bad = 0;
+      for (int r = 0; r < Hb; r++) bad += M[r] == 0;
+      if (cc == 0 || std::memcmp(X, BX, (size_t)Hb * sizeof(double)) != 0)
+        for (int r = 0; r < Hb; r++) bad += !near(ax * (r / k) + bx0, X[r]);
+      for (int r = 0; r < Hb; r++)
+        if (r < k || !(Y[r] == Y[r - k])) bad += !near(ay * ((double)cc * k + r % k) + by0, Y[r]);
+      ok = bad == 0;
+    }
     if (ok) {
       g.geo_k = k;
       g.geo_L = L;
@@ -832,6 +934,7 @@ struct Batch::Impl {
   cudaEvent_t ev_up = nullptr;
   int* d_ready = nullptr;
   void* early = nullptr;  // streamed frames, their image sums, sum scratch and ready flags (pool)
+  std::vector<std::pair<void*, size_t>> touch;  // more host memory that the run's results go to
   bool pool_arena = false;  // the arena comes from the library's memory pool
   // flag t: CUDA-event timing of the stages, summed into the reference's sub-function slots
   // (output 10, timedmainiteration.cpp:45-143 and task.cpp:293-356); the interval from a mark to the
@@ -902,14 +1005,14 @@ Batch::~Batch() {
   for (cudaEvent_t e : d->fevents) cudaEventDestroy(e);
   if (d->ev_cycle) cudaEventDestroy(d->ev_cycle);
   if (d->run_exec) cudaGraphExecDestroy(d->run_exec);
-  if (d->cap_stream) cudaStreamDestroy(d->cap_stream);
+  if (d->cap_stream) give_stream(d->cap_stream, d->device);
   if (d->up_stream) {
     cudaStreamSynchronize(d->up_stream);
     if (d->early) {
       cudaFreeAsync(d->early, d->up_stream);
       cudaStreamSynchronize(d->up_stream);
     }
-    cudaStreamDestroy(d->up_stream);
+    give_stream(d->up_stream, d->device);
   }
   if (d->ev_up) cudaEventDestroy(d->ev_up);
   if (d->arena && !d->external_arena) {
@@ -921,7 +1024,7 @@ Batch::~Batch() {
     }
   }
   if (d->h_counters) cudaFreeHost(d->h_counters);
-  if (d->stream && d->own_stream) cudaStreamDestroy(d->stream);
+  if (d->stream && d->own_stream) give_stream(d->stream, d->device);
   delete d;
 }
 
@@ -1114,7 +1217,8 @@ static int start_frame_uploads(Batch::Impl* b, int device) {
       return fail(SS_ERR_INVALID_ARGUMENT, "streamed frames: group not validated");
     if (!g.frames_dev) bytes += up(g.frame_bytes);
   }
-  SS_CK(cudaStreamCreateWithFlags(&b->up_stream, cudaStreamNonBlocking));
+  b->device = device;
+  SS_CK(take_stream(&b->up_stream));
   SS_CK(cudaEventCreateWithFlags(&b->ev_up, cudaEventDisableTiming));
   cudaMemPool_t pool = work_pool(device);
   if (!pool) return fail(SS_ERR_OUT_OF_MEMORY, "no device memory pool");
@@ -1291,7 +1395,7 @@ int Batch::prepare(int n, const ss_inputs* in, ss_outputs* out, void* external, 
     b->stream = static_cast<cudaStream_t>(borrow_stream);
     b->own_stream = false;
   } else {
-    SS_CK(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
+    SS_CK(take_stream(&b->stream));
     b->own_stream = true;
   }
   // the early buffer was allocated on the upload stream: order it before this stream's work (the
@@ -1325,41 +1429,17 @@ int Batch::prepare(int n, const ss_inputs* in, ss_outputs* out, void* external, 
       SS_CK(stg.put((void*)G.frac, g.frac.data(), hbw * 8));
       SS_CK(stg.put((void*)G.basex, g.bx.data(), hbw * 8));
       SS_CK(stg.put((void*)G.basey, g.by.data(), hbw * 8));
-      if (b->compute == 1) {  // precision 'S' geometry, converted straight into the staging buffer
-        const double* src[3] = {g.frac.data(), g.bx.data(), g.by.data()};
-        const float* dst[3] = {G.frac_f, G.basex_f, G.basey_f};
-        std::vector<float>* keep[3] = {&g.frac_f, &g.bx_f, &g.by_f};
-        for (int a = 0; a < 3; a++) {
-          float* h = static_cast<float*>(stg.take(hbw * 4));
-          if (!h) {
-            keep[a]->resize(hbw);
-            h = keep[a]->data();
-          }
-          for (size_t e = 0; e < hbw; e++) h[e] = (float)src[a][e];
-          SS_CK(cudaMemcpyAsync((void*)dst[a], h, hbw * 4, cudaMemcpyHostToDevice, s));
-        }
-      }
       SS_CK(stg.put((void*)G.base_mask, g.bmask.data(), hbw));
       SS_CK(stg.put((void*)G.min_points, g.minp.data(), g.W * 4));
       if (G.geo_shared) {
         k_set_flag<<<1, 1, 0, s>>>((int*)G.geo_shared);
         k_geo_shared<<<148, 256, 0, s>>>(G.frac, G.basex, G.basey, G.base_mask, g.Hb, g.W, (int*)G.geo_shared);
       }
-      if (G.col_yrange) {  // [min, max] of basey over the valid rows of each block column
-        const double* BY = g.by.data();
-        g.yrange.assign(2 * (size_t)g.W, 0.0f);
-        for (int c = 0; c < g.W; c++) {
-          double lo = INFINITY, hi = -INFINITY;
-          for (int r = 0; r < g.Hb; r++) {
-            const size_t i = (size_t)c * g.Hb + r;
-            if (!g.bmask[i]) continue;
-            lo = std::min(lo, BY[i]);
-            hi = std::max(hi, BY[i]);
-          }
-          g.yrange[2 * c] = (float)lo;
-          g.yrange[2 * c + 1] = (float)hi;
-        }
-        SS_CK(stg.put((void*)G.col_yrange, g.yrange.data(), g.yrange.size() * 4));
+      if (b->compute == 1) {  // precision 'S': FP32 tables and each column's basey range
+        k_geo_single<<<148 * 2, 256, 0, s>>>(G.frac, G.basex, G.basey, hbw, (float*)G.frac_f, (float*)G.basex_f,
+                                             (float*)G.basey_f);
+        k_col_yrange<<<(g.W + 7) / 8, 256, 0, s>>>(G.basey, G.base_mask, g.Hb, g.W, (float*)G.col_yrange);
+        SS_CK(cudaGetLastError());
       }
     }
     const bool streamed = g.early_image != nullptr;  // uploaded by start_frame_uploads
@@ -1645,7 +1725,7 @@ static int prime_attributes(Batch::Impl* b) {
 static int build_run_graph(Batch::Impl* b) {
   int rc = prime_attributes(b);
   if (rc) return rc;
-  if (!b->cap_stream) SS_CK(cudaStreamCreateWithFlags(&b->cap_stream, cudaStreamNonBlocking));
+  if (!b->cap_stream) SS_CK(take_stream(&b->cap_stream));
   cudaStream_t s = b->cap_stream;
   const int nG = (int)b->gd.size();
   // two half-steps per iteration, a line search of up to kTrialCap trials each
@@ -1818,11 +1898,28 @@ int Batch::poll() {
   return 1;
 }
 
+// The host outputs of a batch whose run has been launched (touch_pages).
+static void touch_outputs(Batch::Impl* b) {
+  for (size_t i = 0; i < b->hg.size(); i++) {
+    const HostGroup& g = b->hg[i];
+    const size_t nk = (size_t)(g.W + 1) * g.nF * 8;
+    if (const ss_outputs* o = b->outs[i]) {
+      touch_pages(o->dx_knots, nk);
+      touch_pages(o->dy_knots, nk);
+      touch_pages(o->mask, (size_t)g.Hb * g.fW);
+    }
+  }
+  for (const auto& t : b->touch) touch_pages(t.first, t.second);
+}
+
 int Batch::run() {
+  bool touched = false;
   int rc = start();
   if (rc) return rc;
   for (;;) {
     if ((rc = step())) return rc;
+    if (!touched) touch_outputs(d);
+    touched = true;
     SS_CK(cudaStreamSynchronize(d->stream));
     rc = poll();
     if (rc < 0) return rc;
@@ -2285,8 +2382,10 @@ int estimate_displacements(const ss_recording* rec, ss_recording_outputs* out) {
   }
   Batch b;
   if ((rc = b.prepare(n_sets, ins.data(), nullptr, nullptr, 0))) return rc;
-  if ((rc = b.run())) return rc;
   Batch::Impl* bi = b.d;
+  bi->touch = {{out->dx_knots, (size_t)(W + 1) * n * 8}, {out->dy_knots, (size_t)(W + 1) * n * 8},
+               {out->blocks_used, (size_t)W * n}};
+  if ((rc = b.run())) return rc;
   cudaStream_t s = bi->stream;
   // the recording's outputs on the device: NaN / 0 where no set estimates a frame
   const size_t nk = (size_t)(W + 1) * n, nd = 2 * nk + 3 * (size_t)n, nb = (size_t)n + (size_t)W * n;
@@ -2363,6 +2462,7 @@ static cudaMemPool_t work_pool(int device) {
 struct CallMem {
   std::vector<void*> ptrs;
   cudaStream_t s = nullptr;
+  int dev = 0;  // of s
   cudaMemPool_t pool = nullptr;
   CallMem() = default;
   CallMem(const CallMem&) = delete;
@@ -2371,15 +2471,14 @@ struct CallMem {
     for (void* q : ptrs) cudaFreeAsync(q, s);
     if (s) {
       cudaStreamSynchronize(s);
-      cudaStreamDestroy(s);
+      give_stream(s, dev);
     }
   }
   template <class T>
   T* take(size_t count) {
     if (!s) return nullptr;
     if (!pool) {
-      int dev = 0;
-      if (cudaGetDevice(&dev) != cudaSuccess || !(pool = work_pool(dev))) return nullptr;
+      if (!(pool = work_pool(dev))) return nullptr;
     }
     void* q = nullptr;
     if (cudaMallocFromPoolAsync(&q, std::max<size_t>(1, count) * sizeof(T), pool, s) != cudaSuccess) return nullptr;
@@ -2570,7 +2669,8 @@ int prepare_frames(const ss_prep_frames* p) {
   if (p->frames.location == SS_HOST) per_pass = std::min(per_pass, ((size_t)128 << 20) / (fsz * npx));
   const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)n, per_pass));
   CallMem m;
-  SS_CK(cudaStreamCreateWithFlags(&m.s, cudaStreamNonBlocking));
+  m.dev = p->gpu_device_id;
+  SS_CK(take_stream(&m.s));
   cudaStream_t s = m.s;
   const size_t map_n = map.kmax ? map.start.size() : (size_t)hb * nbk;
   int* d_gather = m.take<int>(map_n);
@@ -2709,7 +2809,8 @@ int reconstruct_frames(const ss_reconstruct* r) {
   const int chunk = (int)std::max<size_t>(1, std::min<size_t>({(size_t)n, (size_t)64, kRingBytes / (iterate * slots)}));
   const size_t px = (size_t)hd * wd, fsz = fr.dtype == SS_F64 ? 8 : 4, osz = o.dtype == SS_F64 ? 8 : 4;
   CallMem m;
-  SS_CK(cudaStreamCreateWithFlags(&m.s, cudaStreamNonBlocking));
+  m.dev = r->gpu_device_id;
+  SS_CK(take_stream(&m.s));
   cudaStream_t s = m.s;
   double* d_bx = m.take<double>(px);
   double* d_by = m.take<double>(px);
@@ -2843,6 +2944,17 @@ int reconstruct_frames(const ss_reconstruct* r) {
       }
     };
     settle();
+    // a part of the chunk's host outputs is touched while each round runs (4 MB take about as long)
+    size_t touched = 0;
+    auto touch_some = [&] {
+      const size_t out_n = o.location == SS_HOST ? osz * fnp : 0, mk_n = r->mask ? fnp : 0, part = size_t(4) << 20;
+      char* ob = static_cast<char*>(const_cast<void*>(o.data)) + osz * (size_t)f0 * np;
+      char* mb = reinterpret_cast<char*>(r->mask) + (size_t)f0 * np;
+      if (touched < out_n) touch_pages(ob + touched, std::min(part, out_n - touched));
+      else if (touched < out_n + mk_n) touch_pages(mb + (touched - out_n), std::min(part, out_n + mk_n - touched));
+      if (touched < out_n) touched = std::min(out_n, touched + part);
+      else touched += part;
+    };
     for (int it = 0; next < F; it += it ? kRcBatch : 1) {  // iterate 0, then kRcBatch at a time
       if (it > kMaxSweeps) return fail(SS_ERR_CUDA, "reconstruct: the energy kept decreasing over 4M sweeps");
       const int nit = it ? kRcBatch : 1;
@@ -2852,6 +2964,7 @@ int reconstruct_frames(const ss_reconstruct* r) {
       energies(F, it, nit);
       SS_CK(cudaGetLastError());
       SS_CK(cudaMemcpyAsync(got.data(), d_energy, got.size() * 4, cudaMemcpyDeviceToHost, s));
+      touch_some();
       SS_CK(cudaStreamSynchronize(s));
       for (int f = 0; f < F; f++) {
         if (limit[f] < 0) continue;
