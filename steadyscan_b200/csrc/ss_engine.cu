@@ -641,7 +641,8 @@ enum RunCounter {
   kCtrRound = 3,      // trial rounds of the graph's current cycle
   kCtrRounds = 4,     // trial rounds run by the graph
   kCtrBound = 5,      // bit 0: the graph stopped at the cycle bound; bit 1: a cycle hit its round bound
-  kCtrWaiting = 6,    // groups whose streamed frames have not arrived (k_join)
+  kCtrWaiting = 6,    // groups whose streamed frames have not arrived (join_groups)
+  kCtrStopped = 7,    // groups whose iterations have ended (their final pass is due or done)
   kCounters = 8
 };
 
@@ -1559,8 +1560,8 @@ constexpr int kFirstRounds = 8, kMinRounds = 3, kMaxRounds = 16;
 // Groups whose streamed frames have arrived (ready flag, written on the upload stream after the
 // frames and their image sum) join the run at the start of the cycle; ctr[kCtrWaiting] counts those
 // still waiting. One CTA.
-__global__ void __launch_bounds__(1024) k_join(GroupCtl* __restrict__ ctl, const int* __restrict__ ready, int n_groups,
-                                               int* __restrict__ ctr) {
+__device__ __forceinline__ void join_groups(GroupCtl* __restrict__ ctl, const int* __restrict__ ready, int n_groups,
+                                            int* __restrict__ ctr) {
   int waiting = 0;
   for (int g = threadIdx.x; g < n_groups; g += blockDim.x) {
     if (ctl[g].phase != kPhWait) continue;
@@ -1576,6 +1577,11 @@ __global__ void __launch_bounds__(1024) k_join(GroupCtl* __restrict__ ctl, const
     for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += sw[w];
     ctr[kCtrWaiting] = t;
   }
+  __syncthreads();
+}
+__global__ void __launch_bounds__(1024) k_join(GroupCtl* __restrict__ ctl, const int* __restrict__ ready, int n_groups,
+                                               int* __restrict__ ctr) {
+  join_groups(ctl, ready, n_groups, ctr);
 }
 
 
@@ -1626,7 +1632,7 @@ static int enqueue_cycle(Batch::Impl* b) {
   b->fmark(10);
   k_iter_sums<<<dim3(kIterSplit, nG), 256, 0, s>>>(b->d_gd, b->d_ctl);
   b->fmark(11);
-  k_iter_end<<<nG, kSolveThreads, 0, s>>>(b->d_gd, b->d_ctl);
+  k_iter_end<<<nG, kSolveThreads, 0, s>>>(b->d_gd, b->d_ctl, nullptr);
   b->fmark(-1);
   b->eval_timed(kFinal);
   k_final<<<nG, kSolveThreads, 0, s>>>(b->d_gd, b->d_ctl, b->d_counters + 1);
@@ -1651,22 +1657,32 @@ static int launch_cycle(Batch::Impl* b) {
 
 // ---------------------------------------------------------------------------------------------
 // The whole run as one CUDA graph: a WHILE node over cycles whose body is the cycle, and inside it
-// (precision 'S') a WHILE node over trial rounds. One-thread control kernels set both conditions
+// (precision 'S') a WHILE node over trial rounds; the final pass follows the loop. One-CTA control kernels
+// build the schedules and set both conditions
 // from the groups' state on the device, so the run needs no host round trip until every group has
 // stopped. Both loops are bounded by counters (cycles by the batch's cycle bound, rounds per cycle
 // by kGraphRounds, after which a search continues in the next cycle).
 
 constexpr int kGraphRounds = 64;
 
+// The schedules of the batch's evaluation launches, as the control kernels of the run graph build them.
+struct SchedArgs {
+  const int* chunk_group;
+  int n_chunks;
+  int* sched;
+};
+
 // Schedule of the next trial round and the condition of the trial-round loop: another round while
-// a frame is searching and the cycle is under its round bound. `first` starts the cycle's count.
+// a frame is searching and the cycle is under its round bound. `first` starts the cycle's count. After
+// the last round, the schedule of the correlation pass.
 __global__ void __launch_bounds__(kSchedThreads) k_sched_rounds(const GroupDesc* __restrict__ gds,
                                                                 const GroupCtl* __restrict__ ctl,
                                                                 const int* __restrict__ frame_group, int n_frames,
                                                                 int n_groups, int* __restrict__ tsched,
                                                                 int* __restrict__ ctr, int first, int slots,
-                                                                cudaGraphConditionalHandle h) {
+                                                                SchedArgs ev, cudaGraphConditionalHandle h) {
   const int tiles = build_trial_schedule(gds, ctl, frame_group, n_frames, n_groups, tsched, slots);
+  __shared__ int s_more;
   if (threadIdx.x == 0) {
     if (first) ctr[kCtrRound] = 0;
     const bool more = tiles > 0 && ctr[kCtrRound] < kGraphRounds;
@@ -1677,18 +1693,33 @@ __global__ void __launch_bounds__(kSchedThreads) k_sched_rounds(const GroupDesc*
       ctr[kCtrBound] |= 2;
     }
     cudaGraphSetConditional(h, more ? 1u : 0u);
+    s_more = more;
   }
+  __syncthreads();
+  if (!s_more) build_schedule<kCorr>(gds, ctl, ev.chunk_group, ev.n_chunks, ev.sched, ev.n_chunks);
 }
 
-// Condition of the cycle loop: another cycle while a group is running, up to `max_cycles`. A cycle
-// in which every running group still waits for its frames does not count toward the bound.
-__global__ void k_cycle_ctl(int* __restrict__ ctr, int n_groups, int max_cycles, cudaGraphConditionalHandle h) {
-  if (threadIdx.x != 0) return;
-  const bool idle = ctr[kCtrWaiting] > 0 && ctr[kCtrWaiting] + ctr[kCtrDone] >= n_groups;
-  const int c = idle ? ctr[kCtrCycles] : ++ctr[kCtrCycles];
-  const bool running = ctr[kCtrDone] < n_groups;
-  if (running && c >= max_cycles) ctr[kCtrBound] |= 1;
-  cudaGraphSetConditional(h, running && c < max_cycles ? 1u : 0u);
+// End of a cycle: the condition of the cycle loop, another cycle while a group is running, up to
+// `max_cycles` (a cycle in which every running group still waits for its frames does not count toward
+// the bound), and the next cycle's start: groups whose frames have arrived join, and the assembly's
+// schedule. One CTA: separate launches of these cost a small run a fifth of its cycle.
+__global__ void __launch_bounds__(kSchedThreads) k_cycle_ctl(const GroupDesc* __restrict__ gds,
+                                                             GroupCtl* __restrict__ ctl, const int* __restrict__ ready,
+                                                             int* __restrict__ ctr, int n_groups, int max_cycles,
+                                                             SchedArgs ev, cudaGraphConditionalHandle h) {
+  __shared__ int s_go;
+  if (threadIdx.x == 0) {
+    const bool idle = ctr[kCtrWaiting] > 0 && ctr[kCtrWaiting] + ctr[kCtrStopped] >= n_groups;
+    const int c = idle ? ctr[kCtrCycles] : ++ctr[kCtrCycles];
+    const bool running = ctr[kCtrStopped] < n_groups;
+    if (running && c >= max_cycles) ctr[kCtrBound] |= 1;
+    s_go = running && c < max_cycles;
+    cudaGraphSetConditional(h, s_go ? 1u : 0u);
+  }
+  __syncthreads();
+  if (!s_go) return;
+  if (ready) join_groups(ctl, ready, n_groups, ctr);
+  build_schedule<kAssemble>(gds, ctl, ev.chunk_group, ev.n_chunks, ev.sched, ev.n_chunks);
 }
 
 // Adds a WHILE node after the work captured so far on `s` and makes it the capture's dependency;
@@ -1741,10 +1772,21 @@ static int build_run_graph(Batch::Impl* b) {
   cudaGraphConditionalHandle h_cycle = 0, h_round = 0;
   SS_CK(cudaGraphConditionalHandleCreate(&h_cycle, top, 1, cudaGraphCondAssignDefault));
   const cudaStreamCaptureMode mode = cudaStreamCaptureModeThreadLocal;
-  // top: counters, the cycle loop, the counters to the host
+  int* sc = b->d_sched;
+  const int nc = b->n_chunks, slots = trial_slots();
+  const SchedArgs ev{b->d_chunk_group, nc, sc};
+  // top: counters, the first cycle's start, the cycle loop, the final pass of every group (their states
+  // stand from the end of their iterations), the counters to the host
   SS_CK(cudaStreamBeginCaptureToGraph(s, top, nullptr, nullptr, 0, mode));
-  cudaMemsetAsync(b->d_counters + kCtrCycles, 0, (kCtrWaiting - kCtrCycles + 1) * sizeof(int), s);
+  cudaMemsetAsync(b->d_counters + kCtrCycles, 0, (kCtrStopped - kCtrCycles + 1) * sizeof(int), s);
+  if (b->d_ready) k_join<<<1, 1024, 0, s>>>(b->d_ctl, b->d_ready, nG, b->d_counters);
+  sched_launch(kAssemble, s, b->d_gd, b->d_ctl, b->d_chunk_group, nc, sc);
   rc = capture_while(s, h_cycle, &body);
+  if (!rc) {
+    sched_launch(kFinal, s, b->d_gd, b->d_ctl, b->d_chunk_group, nc, sc);
+    b->ks.eval(kFinal, b->n_tiles, s, b->d_gd, sc, nc, b->d_ctl, b->max_hb, b->win_bytes);
+    k_final<<<nG, kSolveThreads, 0, s>>>(b->d_gd, b->d_ctl, b->d_counters + kCtrDone);
+  }
   cudaMemcpyAsync(b->h_counters, b->d_counters, kCounters * sizeof(int), cudaMemcpyDeviceToHost, s);
   cudaGraph_t out = nullptr;
   cudaError_t e = cudaStreamEndCapture(s, &out);
@@ -1753,30 +1795,20 @@ static int build_run_graph(Batch::Impl* b) {
   // one cycle
   if (b->ks.round) SS_CK(cudaGraphConditionalHandleCreate(&h_round, body, 0, 0));
   SS_CK(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, mode));
-  int* sc = b->d_sched;
-  const int nc = b->n_chunks;
-  if (b->d_ready) k_join<<<1, 1024, 0, s>>>(b->d_ctl, b->d_ready, nG, b->d_counters);
-  sched_launch(kAssemble, s, b->d_gd, b->d_ctl, b->d_chunk_group, nc, sc);
   b->ks.eval(kAssemble, b->n_tiles, s, b->d_gd, sc, nc, b->d_ctl, b->max_hb, b->win_bytes);
   solve_launch(s, b->d_gd, b->d_ctl, nG);
   if (b->ks.round) {
     k_sched_rounds<<<1, kSchedThreads, 0, s>>>(b->d_gd, b->d_ctl, b->d_frame_group, b->n_frames_total, nG,
-                                               b->d_tsched, b->d_counters, 1, trial_slots(), h_round);
+                                               b->d_tsched, b->d_counters, 1, slots, ev, h_round);
     rc = capture_while(s, h_round, &rounds_body);
-    if (!rc) {
-      sched_launch(kCorr, s, b->d_gd, b->d_ctl, b->d_chunk_group, nc, sc);
-      b->ks.eval(kCorr, b->n_tiles, s, b->d_gd, sc, nc, b->d_ctl, b->max_hb, b->win_bytes);
-    }
+    if (!rc) b->ks.eval(kCorr, b->n_tiles, s, b->d_gd, sc, nc, b->d_ctl, b->max_hb, b->win_bytes);
   } else {
     b->ks.ls(b->n_frames_total, s, b->d_gd, b->d_frame_group, b->d_ctl, b->ls_geo_rows);
   }
   k_after_ls<<<nG, kAfterLsThreads, 0, s>>>(b->d_gd, b->d_ctl);
   k_iter_sums<<<dim3(kIterSplit, nG), 256, 0, s>>>(b->d_gd, b->d_ctl);
-  k_iter_end<<<nG, kSolveThreads, 0, s>>>(b->d_gd, b->d_ctl);
-  sched_launch(kFinal, s, b->d_gd, b->d_ctl, b->d_chunk_group, nc, sc);
-  b->ks.eval(kFinal, b->n_tiles, s, b->d_gd, sc, nc, b->d_ctl, b->max_hb, b->win_bytes);
-  k_final<<<nG, kSolveThreads, 0, s>>>(b->d_gd, b->d_ctl, b->d_counters + kCtrDone);
-  k_cycle_ctl<<<1, 32, 0, s>>>(b->d_counters, nG, max_cycles, h_cycle);
+  k_iter_end<<<nG, kSolveThreads, 0, s>>>(b->d_gd, b->d_ctl, b->d_counters + kCtrStopped);
+  k_cycle_ctl<<<1, kSchedThreads, 0, s>>>(b->d_gd, b->d_ctl, b->d_ready, b->d_counters, nG, max_cycles, ev, h_cycle);
   e = cudaStreamEndCapture(s, &out);
   if (rc) return rc;
   if (e != cudaSuccess) return fail(SS_ERR_CUDA, std::string("run graph cycle: ") + cudaGetErrorString(e));
@@ -1785,7 +1817,7 @@ static int build_run_graph(Batch::Impl* b) {
     SS_CK(cudaStreamBeginCaptureToGraph(s, rounds_body, nullptr, nullptr, 0, mode));
     b->ks.round(b->n_trial_tiles, s, b->d_gd, b->d_tsched, b->n_frames_total, nG, b->d_ctl, b->win_bytes);
     k_sched_rounds<<<1, kSchedThreads, 0, s>>>(b->d_gd, b->d_ctl, b->d_frame_group, b->n_frames_total, nG,
-                                               b->d_tsched, b->d_counters, 0, trial_slots(), h_round);
+                                               b->d_tsched, b->d_counters, 0, slots, ev, h_round);
     e = cudaStreamEndCapture(s, &out);
     if (e != cudaSuccess) return fail(SS_ERR_CUDA, std::string("run graph rounds: ") + cudaGetErrorString(e));
   }
@@ -1878,10 +1910,10 @@ int Batch::poll() {
     b->graph_run = false;
     b->cycles = c[kCtrCycles];
     b->rounds = b->ks.round ? c[kCtrRounds] : c[kCtrCycles];
-    // per cycle: schedules and evaluation passes, the solve (5), after-ls, iteration end (2), final,
-    // cycle control, and the line search (precision 'D') or the first round schedule and the
-    // correlation pass (precision 'S'); two launches per trial round
-    b->launches = b->ks.round ? 17 * c[kCtrCycles] + 2 * c[kCtrRounds] : 15 * c[kCtrCycles];
+    // once: the first assembly schedule, the final pass (3), the join of streamed frames; per cycle: the
+    // assembly, the solve (5), after-ls, iteration end (2), cycle control, and the line search (precision
+    // 'D') or the first round schedule and the correlation pass (precision 'S'); two per trial round
+    b->launches = (b->ks.round ? 12 * c[kCtrCycles] + 2 * c[kCtrRounds] : 11 * c[kCtrCycles]) + (b->d_ready ? 5 : 4);
     if (c[kCtrBound] & 1) return fail(SS_ERR_CUDA, "alignment did not finish within the iteration bound");
     b->state = 3;
     int rc = finish_run(b);
@@ -2274,7 +2306,7 @@ int Server::step() {
   }
   k_after_ls<<<nG, kAfterLsThreads, 0, s>>>(v->d_gd, v->d_ctl);
   k_iter_sums<<<dim3(kIterSplit, nG), 256, 0, s>>>(v->d_gd, v->d_ctl);
-  k_iter_end<<<nG, kSolveThreads, 0, s>>>(v->d_gd, v->d_ctl);
+  k_iter_end<<<nG, kSolveThreads, 0, s>>>(v->d_gd, v->d_ctl, nullptr);
   sched_launch(kFinal, s, v->d_gd, v->d_ctl, v->d_chunk_group, nc, sc);
   v->ks.eval(kFinal, v->n_tiles, s, v->d_gd, sc, nc, v->d_ctl, v->max_hb, v->win_bytes);
   k_final<<<nG, kSolveThreads, 0, s>>>(v->d_gd, v->d_ctl, v->d_counters + 1);

@@ -975,8 +975,9 @@ __global__ void __launch_bounds__(256) k_iter_sums(const GroupDesc* __restrict__
 }
 
 // End of an iteration (task.cpp:281-373) for groups in kPhIterEnd, after k_eval<kCorr> and
-// k_iter_sums.
-__global__ void __launch_bounds__(kSolveThreads) k_iter_end(const GroupDesc* __restrict__ gds, GroupCtl* __restrict__ ctl) {
+// k_iter_sums. `stopped` (may be null) counts the groups whose iterations end.
+__global__ void __launch_bounds__(kSolveThreads) k_iter_end(const GroupDesc* __restrict__ gds, GroupCtl* __restrict__ ctl,
+                                                            int* __restrict__ stopped) {
   const GroupDesc& G = gds[blockIdx.x];
   GroupCtl& C = ctl[blockIdx.x];
   if (C.phase != kPhIterEnd) return;
@@ -1094,7 +1095,10 @@ __global__ void __launch_bounds__(kSolveThreads) k_iter_end(const GroupDesc* __r
       if (frame_active(G, f, 0)) G.kdiff[i] = G.kmask[i];
     }
     __syncthreads();
-    if (t == 0) C.phase = kPhFinal;
+    if (t == 0) {
+      C.phase = kPhFinal;
+      if (stopped) atomicAdd(stopped, 1);
+    }
   } else if (t == 0) {
     C.iteration = it + 1;
     C.shift = 0;
