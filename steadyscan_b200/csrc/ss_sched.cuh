@@ -181,7 +181,11 @@ __device__ __forceinline__ bool fetch_tile(int* __restrict__ sched, int cap, int
 // each standing for the group's W tiles (one block column each); a tile's warps take its frames in
 // turn. Each tile stages one template window for its frames, so tiles of 32 frames spend a quarter
 // of the staging of tiles of 8 (512x512 frames, 2-line knots, groups of 64: trial rounds 85 ms with
-// 32 frames per tile, 94 ms with 8).
+// 32 frames per tile, 94 ms with 8). A round of few frames takes tiles of 16 or 8 frames, 8 being a
+// column for each warp: tiles of 32 are taken from 6 waves of the `slots` resident CTAs on, tiles of 16
+// from 4; below that the last wave, part filled, costs more than the staging (trial rounds of a ragged
+// batch of 24 groups: 91 ms with tiles of 32 throughout, 84 with the lines at 3 and 2 waves, 77.6 at 6 and
+// 4, 76.6 at 12 and 8; of 31 groups of 64 frames of 512 x 512: 47.4, 44.7, 44.7 and 45.7).
 
 #ifndef SS_TRIAL_TILE_FRAMES
 #define SS_TRIAL_TILE_FRAMES 32
@@ -189,7 +193,7 @@ __device__ __forceinline__ bool fetch_tile(int* __restrict__ sched, int cap, int
 constexpr int kTrialTileFrames = SS_TRIAL_TILE_FRAMES;
 constexpr int kTrialTileMin = 8;
 __device__ __forceinline__ int trial_tile_frames(long long columns, int slots) {
-  return columns >= 96LL * slots ? kTrialTileFrames : columns >= 32LL * slots ? 16 : kTrialTileMin;
+  return columns >= 192LL * slots ? kTrialTileFrames : columns >= 64LL * slots ? 16 : kTrialTileMin;
 }
 
 // Buffer: header, list[nf] (batch frame index of each searching frame), first[ng] and end[ng] (each
