@@ -375,7 +375,9 @@ __device__ __forceinline__ void trial_pairs16(const GroupDesc& G, size_t coli, c
 // Correlation sums (kCsSumD .. kCsFrDI) of one block column whose mask and difference-image knots
 // agree, in the reference's definitions (task_correlation.cu:16-60, swapped difference image D'),
 // and for the final pass also the SSD at the mask knots and the mask output. The leading run of
-// valid pixels follows the row order: within a 64-row step lane L holds rows 2L and 2L + 1.
+// valid pixels follows the row order: within a 64-row step lane L holds rows 2L and 2L + 1. While the
+// run holds its sums are those over all valid pixels, so they are formed only in the step in which it
+// ends: the sums so far plus that step's pixels before the first invalid one.
 template <class FrameT, int MODE>
 __device__ __forceinline__ void corr_pairs(const GroupDesc& G, size_t coli, const PairCol& pc, const PairWin& w,
                                            double (&out)[kCsStride], int& cnt_out, uint8_t* mask_out) {
@@ -386,10 +388,10 @@ __device__ __forceinline__ void corr_pairs(const GroupDesc& G, size_t coli, cons
   const FrameT* col = reinterpret_cast<const FrameT*>(G.image) + coli;
   const int steps = G.Hb >> 6;
   const unsigned lt = (1u << lane) - 1u;
-  float2 sumd = f2(0.f), sn = f2(0.f), sd = f2(0.f), sdd = f2(0.f), si = f2(0.f), sii = f2(0.f), sdi = f2(0.f),
-         fd = f2(0.f), fi = f2(0.f), fdd = f2(0.f), fii = f2(0.f), fdi = f2(0.f), fssd = f2(0.f);
+  float2 fd = f2(0.f), fi = f2(0.f), fdd = f2(0.f), fii = f2(0.f), fdi = f2(0.f), fssd = f2(0.f);
+  float sn = 0.f, sd = 0.f, sdd = 0.f, si = 0.f, sii = 0.f, sdi = 0.f;  // of the leading run, once it has ended
   int cnt = 0;
-  bool run = true;
+  bool run = true;  // the same in every lane
   float2 j = pc.j0;
   const float2 dj = f2(pc.dj);
   typename PL::W ring[kPrefetchCorr];
@@ -416,25 +418,28 @@ __device__ __forceinline__ void corr_pairs(const GroupDesc& G, size_t coli, cons
       const float2 diff = sub2(img, wI);          // differenceImage at valid pixels
       float2 dp = sub2(img, diff);                // after d_swapWIDiff
       dp = f2(mA ? dp.x : 0.f, mB ? dp.y : 0.f);
-      sumd = add2(sumd, dp);
       const float2 im = f2(mA ? img.x : 0.f, mB ? img.y : 0.f);
+      if (run) {
+        const unsigned bothv = __ballot_sync(0xffffffffu, mA && mB);
+        if (bothv != 0xffffffffu) {  // the run ends in this step
+          run = false;
+          const bool inA = (bothv & lt) == lt && mA, inB = inA && mB;
+          const float2 ds = f2(inA ? dp.x : 0.f, inB ? dp.y : 0.f), is = f2(inA ? img.x : 0.f, inB ? img.y : 0.f);
+          const float2 e = add2(fd, ds), ee = fma2(ds, ds, fdd), g = add2(fi, is), gg = fma2(is, is, fii),
+                       eg = fma2(ds, is, fdi);
+          sn = (float)(2 * t + (inA ? 1 : 0) + (inB ? 1 : 0));
+          sd = e.x + e.y;
+          sdd = ee.x + ee.y;
+          si = g.x + g.y;
+          sii = gg.x + gg.y;
+          sdi = eg.x + eg.y;
+        }
+      }
       fd = add2(fd, dp);
       fi = add2(fi, im);
       fdd = fma2(dp, dp, fdd);
       fii = fma2(im, im, fii);
       fdi = fma2(dp, im, fdi);
-      const unsigned bothv = __ballot_sync(0xffffffffu, mA && mB);
-      const bool pre = run && (bothv & lt) == lt;
-      const bool inA = pre && mA, inB = inA && mB;
-      run = run && bothv == 0xffffffffu;
-      const float2 ds = f2(inA ? dp.x : 0.f, inB ? dp.y : 0.f);
-      const float2 is = f2(inA ? img.x : 0.f, inB ? img.y : 0.f);
-      sn = add2(sn, f2(inA ? 1.f : 0.f, inB ? 1.f : 0.f));
-      sd = add2(sd, ds);
-      sdd = fma2(ds, ds, sdd);
-      si = add2(si, is);
-      sii = fma2(is, is, sii);
-      sdi = fma2(ds, is, sdi);
       if (MODE == kFinal) {
         const float2 dm = f2(mA ? diff.x : 0.f, mB ? diff.y : 0.f);
         fssd = fma2(dm, dm, fssd);
@@ -443,15 +448,23 @@ __device__ __forceinline__ void corr_pairs(const GroupDesc& G, size_t coli, cons
       }
     }
   }
+  if (run) {
+    sn = (float)(2 * steps);
+    sd = fd.x + fd.y;
+    sdd = fdd.x + fdd.y;
+    si = fi.x + fi.y;
+    sii = fii.x + fii.y;
+    sdi = fdi.x + fdi.y;
+  }
   cnt_out = warp_sum(cnt);
-  out[kCsSumD] = (double)warp_sumf(sumd.x + sumd.y);
-  out[kCsSetN] = (double)warp_sumf(sn.x + sn.y);
-  out[kCsSetD] = (double)warp_sumf(sd.x + sd.y);
-  out[kCsSetDD] = (double)warp_sumf(sdd.x + sdd.y);
-  out[kCsSetI] = (double)warp_sumf(si.x + si.y);
-  out[kCsSetII] = (double)warp_sumf(sii.x + sii.y);
-  out[kCsSetDI] = (double)warp_sumf(sdi.x + sdi.y);
+  out[kCsSetN] = (double)warp_sumf(sn);
+  out[kCsSetD] = (double)warp_sumf(sd);
+  out[kCsSetDD] = (double)warp_sumf(sdd);
+  out[kCsSetI] = (double)warp_sumf(si);
+  out[kCsSetII] = (double)warp_sumf(sii);
+  out[kCsSetDI] = (double)warp_sumf(sdi);
   out[kCsFrD] = (double)warp_sumf(fd.x + fd.y);
+  out[kCsSumD] = out[kCsFrD];  // (masked pixels are zero)
   out[kCsFrI] = (double)warp_sumf(fi.x + fi.y);
   out[kCsFrDD] = (double)warp_sumf(fdd.x + fdd.y);
   out[kCsFrII] = (double)warp_sumf(fii.x + fii.y);
