@@ -2942,9 +2942,10 @@ int reconstruct_frames(const ss_reconstruct* r) {
           k_rc_pushgrid<float><<<g, 256, 0, s>>>(b, d_data, f0, F, st, ph, d_bx, d_by, d_tf, d_pk, d_dxk, d_dyk);
       }
     }
-    k_rc_mask<<<g, 256, 0, s>>>(b, F);
-    k_rc_coef<<<g, 256, 0, s>>>(b, F, regfac, vf2);
-    k_rc_count<<<dim3(std::max(1, g / F), F), 256, 0, s>>>(b, d_count);
+    const dim3 fgrid(std::max(1, g / F), F);
+    k_rc_mask<<<fgrid, 256, 0, s>>>(b);
+    k_rc_coef<<<fgrid, 256, 0, s>>>(b, regfac, vf2);
+    k_rc_count<<<fgrid, 256, 0, s>>>(b, d_count);
     SS_CK(cudaGetLastError());
     // the vectors below are the sources and targets of copies on s: each round waits for its copies
     std::vector<int> count(F), limit(F), skip(F), slot(F, -1), iters(F, 0), swept(F, 0), target(F, 0);

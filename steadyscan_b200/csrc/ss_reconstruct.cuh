@@ -155,82 +155,76 @@ __global__ void k_rc_fill_int(int* p, size_t n, int v) {
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) p[e] = v;
 }
 
-// ww entry of the pair (p, q), q - p one of the stencil offsets or their negatives (0 otherwise).
-__device__ __forceinline__ double rc_ww(const double* __restrict__ ww, int th, int np, int p, int q) {
-  const int lo = p < q ? p : q, d = p < q ? q - p : p - q;
-  if (lo < 0 || lo + d >= np) return 0.0;
-  int s = -1;
-  if (d == 0) s = 0;
-  else if (d == 1) s = 1;
-  else if (d == th - 1) s = 2;
-  else if (d == th) s = 3;
-  else if (d == th + 1) s = 4;
-  return s < 0 ? 0.0 : ww[(size_t)s * np + lo];
-}
+// Stencil plane of the pair (p, p + th - 1): NE, or S where the template has two rows and the offsets
+// fall together.
+__device__ __forceinline__ int rc_ne(int th) { return th == 2 ? 1 : 2; }
 
-// Mask (column sums of ww > 0 and a finite first guess) and the first iterate of every pixel.
-__global__ void __launch_bounds__(256) k_rc_mask(RcBufs b, int nf) {
-  const size_t total = (size_t)b.np * nf;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-    const int f = (int)(e / b.np), p = (int)(e - (size_t)f * b.np);
-    const double* ww = b.ww + (size_t)f * b.np * kRcStencil;
-    const int th = b.th;
-    const int nb[9] = {p, p - 1, p + 1, p - th + 1, p + th - 1, p - th, p + th, p - th - 1, p + th + 1};
-    double s = 0.0;
-#pragma unroll
-    for (int j = 0; j < 9; j++) s += rc_ww(ww, th, b.np, p, nb[j]);
+// Mask (column sums of ww > 0 and a finite first guess) and the first iterate of every pixel. Grid:
+// (blocks, frames).
+__global__ void __launch_bounds__(256) k_rc_mask(RcBufs b) {
+  const int f = blockIdx.y, th = b.th, np = b.np, ne = rc_ne(th);
+  const double* ww = b.ww + (size_t)f * np * kRcStencil;
+  const double *S = ww + np, *NE = ww + (size_t)ne * np, *E = ww + (size_t)3 * np, *SE = ww + (size_t)4 * np;
+  float* x = rc_iterate(b, 0, f);
+  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < np; p += gridDim.x * blockDim.x) {
+    double s = ww[p];  // (no entry is negative)
+    if (p >= 1) s += S[p - 1];
+    if (p + 1 < np) s += S[p];
+    if (p >= th - 1) s += NE[p - th + 1];
+    if (p + th - 1 < np) s += NE[p];
+    if (p >= th) s += E[p - th];
+    if (p + th < np) s += E[p];
+    if (p >= th + 1) s += SE[p - th - 1];
+    if (p + th + 1 < np) s += SE[p];
+    const size_t e = (size_t)f * np + p;
     const float iv = b.z[e] / b.cnt[e];
     b.mask[e] = (s > 0.0 && !isnan(iv)) ? 1 : 0;
-    rc_iterate(b, 0, f)[rc_place(b, p % th, p / th)] = isnan(iv) ? 0.0f : iv;
+    const int c = p / th;
+    x[rc_place(b, p - c * th, c)] = isnan(iv) ? 0.0f : iv;
   }
 }
 
-// Q(p, q) of the masked system: ww + regfac GtG (vertical pairs vfac^2), rows and columns of
-// unmasked pixels zero. Diagonal for q == p.
-__device__ __forceinline__ double rc_q(const RcBufs& b, const double* ww, const uint8_t* mk, int p, int q, double regfac,
-                                       double vf2) {
-  if (!mk[p] || !mk[q]) return 0.0;
-  const int th = b.th, r = p % th, c = p / th;
-  double reg = 0.0;
-  if (q == p) {
-    const int nh = (c > 0) + (c < b.tw - 1), nv = (r > 0) + (r < th - 1);
-    reg = regfac * ((double)nh + (double)nv * vf2);
-  } else if ((q == p + 1 && r < th - 1) || (q == p - 1 && r > 0)) {
-    reg = -regfac * vf2;
-  } else if (q == p + th || q == p - th) {
-    reg = -regfac;
-  }
-  return rc_ww(ww, th, b.np, p, q) + reg;
-}
-
-// FP32 coefficients of every pixel: the eight neighbour terms and L; and Le.
-__global__ void __launch_bounds__(256) k_rc_coef(RcBufs b, int nf, double regfac, double vf2) {
-  const size_t total = (size_t)b.np * nf;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-    const int f = (int)(e / b.np), p = (int)(e - (size_t)f * b.np);
-    const double* ww = b.ww + (size_t)f * b.np * kRcStencil;
-    const uint8_t* mk = b.mask + (size_t)f * b.np;
-    const int th = b.th, np = b.np, i = p + 1;  // 1-based, as the finders
-    const float R = (float)rc_q(b, ww, mk, p, p, regfac, vf2);
+// FP32 coefficients of every pixel: the eight neighbour terms and L; and Le. Q(p, q) of the masked system
+// is ww + regfac GtG (vertical pairs vfac^2) with the rows and columns of unmasked pixels zero. Grid:
+// (blocks, frames).
+__global__ void __launch_bounds__(256) k_rc_coef(RcBufs b, double regfac, double vf2) {
+  const int f = blockIdx.y, th = b.th, tw = b.tw, np = b.np, ne = rc_ne(th);
+  const double* ww = b.ww + (size_t)f * np * kRcStencil;
+  const double *S = ww + np, *NE = ww + (size_t)ne * np, *E = ww + (size_t)3 * np, *SE = ww + (size_t)4 * np;
+  const uint8_t* mk = b.mask + (size_t)f * np;
+  const double rh = -regfac, rv = -__dmul_rn(regfac, vf2);
+  const size_t plane = 4 * (size_t)b.nq;
+  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < np; p += gridDim.x * blockDim.x) {
+    const int c = p / th, r = p - c * th;
     // (the entries of a quarter plane past the template's last row or column are never read)
-    float* cf = b.coef + (size_t)f * kRcTerms * 4 * b.nq + rc_place(b, p % th, p / th);
-    const size_t plane = 4 * (size_t)b.nq;
-    // N NE E SE S SW W NW (steady_scan.m:677-723), 1-based candidates and their bounds
-    const int cand[8] = {i - 1, i + th - 1, i + th, i + th + 1, i + 1, i - th + 1, i - th, i - th - 1};
-    const bool ok[8] = {(i - 1) % th != 0, ((i + th - 1) % th != 0) && (i + th - 1 < np), i + th <= np,
-                        (i % th != 0) && (i + th + 1 < np), i % th != 0, (i % th != 0) && (i - th + 1 > 0),
-                        i - th > 0, i - th - 1 > 0};
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-      float t = 0.0f;
-      if (R != 0.0f && ok[j]) t = (float)rc_q(b, ww, mk, p, cand[j] - 1, regfac, vf2) / R;
-      cf[j * plane] = t;
+    float* cf = b.coef + (size_t)f * kRcTerms * plane + rc_place(b, r, c);
+    const bool m = mk[p] != 0;
+    float R = 0.0f;
+    if (m) {
+      const int nh = (c > 0) + (c < tw - 1), nv = (r > 0) + (r < th - 1);
+      R = (float)__dadd_rn(ww[p], __dmul_rn(regfac, (double)nh + (double)nv * vf2));
     }
-    const float lf = mk[p] ? (float)b.wy[e] : 0.0f;
+    // the term of neighbour q within the reference's finders' bounds (steady_scan.m:677-723), its stencil
+    // entry w and regulariser
+    auto term = [&](int j, bool ok, int q, const double* w, int at, double reg) {
+      float t = 0.0f;
+      if (R != 0.0f && ok) t = (mk[q] ? (float)__dadd_rn(w[at], reg) : 0.0f) / R;
+      cf[j * plane] = t;
+    };
+    // N NE E SE S SW W NW; the finders' 1-based bounds (p + 1 = their index)
+    term(0, r > 0, p - 1, S, p - 1, rv);
+    term(1, r > 0 && p + th < np, p + th - 1, NE, p, 0.0);
+    term(2, p + th < np, p + th, E, p, rh);
+    term(3, r < th - 1 && p + th + 2 < np, p + th + 1, SE, p, 0.0);
+    term(4, r < th - 1, p + 1, S, p, rv);
+    term(5, r < th - 1 && p >= th - 1, p - th + 1, NE, p - th + 1, 0.0);
+    term(6, p >= th, p - th, E, p - th, rh);
+    term(7, p >= th + 1, p - th - 1, SE, p - th - 1, 0.0);
+    const float lf = m ? (float)b.wy[(size_t)f * np + p] : 0.0f;
     float L = lf / R;
     if (!isfinite(L)) L = 0.0f;
     cf[8 * plane] = L;
-    b.le[e] = lf;
+    b.le[(size_t)f * np + p] = lf;
   }
 }
 
@@ -287,10 +281,11 @@ __global__ void __launch_bounds__(256) k_rc_linear(RcBufs b, int it0, int nit, i
                                rc_iterate(b, sl.w, f)};
   const int per = (np + kRcParts - 1) / kRcParts, a = blockIdx.x * per, e = min(np, a + per);
   float ls[kRcBatch] = {};
+  int c = (a + (int)threadIdx.x) / th, r = a + (int)threadIdx.x - c * th;
   for (int p = a + threadIdx.x; p < e; p += blockDim.x) {
-    const int c = p / th, r = p - c * th;
-    const size_t at = rc_place(b, r, c);
+    const int at = ((r & 1) * 2 + (c & 1)) * b.nq + (r >> 1) + b.rh * (c >> 1);  // (4 nq < 2^31)
     const float l = le[p];  // zero at unmasked pixels
+    for (r += blockDim.x; r >= th; r -= th) c++;
 #pragma unroll
     for (int k = 0; k < kRcBatch; k++)
       if (k < nit) ls[k] = fmaf(l, xs[k][at], ls[k]);
@@ -322,7 +317,7 @@ __global__ void __launch_bounds__(256) k_rc_quadratic(RcBufs b, int it0, int nit
   const size_t nq = b.nq;
   const double* ww = b.ww + (size_t)f * np * kRcStencil;
   const uint8_t* mk = b.mask + (size_t)f * np;
-  const int s_ne = th == 2 ? 1 : 2;  // (offset th - 1 is S there)
+  const int s_ne = rc_ne(th);
   double qs[kRcBatch] = {};
   for (int k = blockIdx.x * 256 + threadIdx.x; k < b.nq; k += kRcParts * 256) {
     const int j = k / rh, i = k - j * rh, r0 = 2 * i, c0 = 2 * j;
