@@ -311,9 +311,16 @@ static void give_stream(cudaStream_t s, int dev) {
 }
 
 // Has the pages of a host output in place before its copy arrives (the bytes stay as they are): done
-// while the GPU works, since touching fresh pages costs as much as the copy.
+// while the GPU works, since touching fresh pages costs as much as the copy. Pageable memory only:
+// pinned pages are in place, and a device address is the copy's to judge.
 static void touch_pages(void* p, size_t n) {
   if (!p || n < 65536) return;
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  if (at.type != cudaMemoryTypeUnregistered) return;
   volatile char* c = static_cast<volatile char*>(p);
   for (size_t o = 0; o < n; o += 4096) c[o] = c[o];
   c[n - 1] = c[n - 1];
