@@ -306,10 +306,12 @@ __global__ void __launch_bounds__(256) k_rc_linear(RcBufs b, int it0, int nit, i
 // Quadratic energy terms of those iterates: FP64 sums of x_p (Q x)_p over masked p, each pair of pixels
 // once. A thread takes a 2 x 2 quad, the same place of the four quarter planes, so that consecutive
 // lanes read consecutive floats of an iterate, a quad's 11 samples are converted once each, and its 20
-// stencil entries (five times an iterate's bytes) serve nit iterates: 376 us for four iterates of 64
-// frames of 512 x 512, with the linear terms 506; one iterate at a time took 4 x 125 with a thread and
-// 20 conversions per pixel. kRcParts CTAs per frame.
-__global__ void __launch_bounds__(256) k_rc_quadratic(RcBufs b, int it0, int nit, int4 sl, const int* __restrict__ limit,
+// stencil entries (five times an iterate's bytes) serve nit iterates. Bound: load latency at 16 warps
+// per SM (128 registers); so no load waits for another or for a branch, and the next iterate's samples
+// are under way while one is summed. Four iterates of 64 frames of 512 x 512 (147 us of HBM time):
+// 243 us; 376 with each load under its own bounds check. One iterate at a time, with a thread and 20
+// conversions per pixel, took 4 x 125. kRcParts CTAs per frame.
+__global__ void __launch_bounds__(256, 2) k_rc_quadratic(RcBufs b, int it0, int nit, int4 sl, const int* __restrict__ limit,
                                                       double regfac, double vf2) {
   const int f = blockIdx.y;
   if (limit[f] < it0 + nit - 1) return;
@@ -318,18 +320,54 @@ __global__ void __launch_bounds__(256) k_rc_quadratic(RcBufs b, int it0, int nit
   const double* ww = b.ww + (size_t)f * np * kRcStencil;
   const uint8_t* mk = b.mask + (size_t)f * np;
   const int s_ne = rc_ne(th);
+  const bool paired = (th & 1) == 0;  // then every column, plane and frame of ww starts on 16 bytes
   double qs[kRcBatch] = {};
   for (int k = blockIdx.x * 256 + threadIdx.x; k < b.nq; k += kRcParts * 256) {
     const int j = k / rh, i = k - j * rh, r0 = 2 * i, c0 = 2 * j;
-    auto masked = [&](int r, int c) {
-      return (unsigned)r < (unsigned)th && (unsigned)c < (unsigned)tw && mk[(size_t)c * th + r] != 0;
-    };
+    const bool up = r0 > 0, down = r0 + 2 < th, low = r0 + 1 < th, right = c0 + 2 < tw, mid = c0 + 1 < tw;
+    // Every load is unconditional, from a clamped place, and its value selected afterwards, so that the
+    // loads of a quad are in flight together.
+    // The stencil entries of the quad's pixels, two rows at a time.
+    double2 w[2][kRcStencil];
+    const size_t p0 = (size_t)c0 * th + r0, p1 = mid ? p0 + th : p0;
+    if (paired) {
+#pragma unroll
+      for (int s = 0; s < kRcStencil; s++) {
+        const double* wp = ww + (size_t)(s == 2 ? s_ne : s) * np;
+        w[0][s] = *reinterpret_cast<const double2*>(wp + p0);
+        w[1][s] = *reinterpret_cast<const double2*>(wp + p1);
+      }
+    } else {
+#pragma unroll
+      for (int s = 0; s < kRcStencil; s++) {
+        const double* wp = ww + (size_t)(s == 2 ? s_ne : s) * np;
+        w[0][s] = make_double2(wp[p0], wp[p0 + low]);
+        w[1][s] = make_double2(wp[p1], wp[p1 + low]);
+      }
+    }
     // masks of the quad and its neighbours: rows r0 - 1 .. r0 + 2, columns c0 .. c0 + 2
+    const bool row_in[4] = {up, true, low, down}, col_in[3] = {true, mid, right};
     bool m[4][3];
 #pragma unroll
-    for (int a = 0; a < 4; a++)
+    for (int e = 0; e < 3; e++)
 #pragma unroll
-      for (int e = 0; e < 3; e++) m[a][e] = masked(r0 - 1 + a, c0 + e);
+      for (int a = 0; a < 4; a++) {
+        const bool in = row_in[a] && col_in[e];
+        m[a][e] = (mk[in ? p0 + (size_t)e * th + a - 1 : p0] != 0) & in;
+      }
+    // iterate t's samples of the quad and its neighbours (past the last of nit, the first's again)
+    const int rt = right ? rh : 0, dn = down ? 1 : 0;
+    auto samples = [&](int t, float (&o)[11]) {
+      const int slot = t >= nit ? sl.x : t == 0 ? sl.x : t == 1 ? sl.y : t == 2 ? sl.z : sl.w;
+      const float* A = rc_iterate(b, slot, f) + k;
+      const float *B = A + nq, *C = A + 2 * nq, *D = A + 3 * nq;
+      o[0] = A[0], o[1] = B[0], o[2] = C[0], o[3] = D[0], o[4] = A[rt], o[5] = C[rt], o[6] = A[dn], o[7] = B[dn];
+      o[8] = A[rt + dn], o[9] = D[up ? -1 : 0], o[10] = C[up ? rt - 1 : rt];
+    };
+    const bool in_x[11] = {true, mid,          low,           low && mid, right,      right && low,
+                           down, down && mid, down && right, up && mid,  up && right};
+    float x[2][11];
+    samples(0, x[0]);
     // Q(p, q) of the quad's pixels (r0 + dr, c0 + dc) with themselves and their S, NE, E, SE neighbours
     double q[2][2][kRcStencil];
 #pragma unroll
@@ -338,29 +376,25 @@ __global__ void __launch_bounds__(256) k_rc_quadratic(RcBufs b, int it0, int nit
       for (int dc = 0; dc < 2; dc++) {
         double* v = q[dr][dc];
         const int r = r0 + dr, c = c0 + dc;
-#pragma unroll
-        for (int s = 0; s < kRcStencil; s++) v[s] = 0.0;
-        if (!m[1 + dr][dc]) continue;
-        const size_t p = (size_t)c * th + r;
+        const bool own = m[1 + dr][dc];
+        auto at = [&](int s) { return dr ? w[dc][s].y : w[dc][s].x; };
         const int nh = (c > 0) + (c < tw - 1), nv = (r > 0) + (r < th - 1);
-        v[0] = ww[p] + regfac * ((double)nh + (double)nv * vf2);
-        if (m[2 + dr][dc]) v[1] = ww[(size_t)np + p] - regfac * vf2;
+        v[0] = own ? at(0) + regfac * ((double)nh + (double)nv * vf2) : 0.0;
+        v[1] = own && m[2 + dr][dc] ? at(1) - regfac * vf2 : 0.0;
         if (th == 2) v[1] += v[1];  // (p + 1 and p + th - 1 are both summed there)
-        if (m[dr][dc + 1]) v[2] = ww[(size_t)s_ne * np + p];
-        if (m[1 + dr][dc + 1]) v[3] = ww[(size_t)3 * np + p] - regfac;
-        if (m[2 + dr][dc + 1]) v[4] = ww[(size_t)4 * np + p];
+        v[2] = own && m[dr][dc + 1] ? at(2) : 0.0;
+        v[3] = own && m[1 + dr][dc + 1] ? at(3) - regfac : 0.0;
+        v[4] = own && m[2 + dr][dc + 1] ? at(4) : 0.0;
       }
-    const bool up = r0 > 0, down = r0 + 2 < th, low = r0 + 1 < th, right = c0 + 2 < tw, mid = c0 + 1 < tw;
 #pragma unroll
     for (int t = 0; t < kRcBatch; t++) {
-      if (t >= nit) break;
-      const float* x = rc_iterate(b, t == 0 ? sl.x : t == 1 ? sl.y : t == 2 ? sl.z : sl.w, f) + k;
-      const float *A = x, *B = x + nq, *C = x + 2 * nq, *D = x + 3 * nq;
-      // rows r0 - 1 .. r0 + 2, columns c0 .. c0 + 2
-      const double a0 = A[0], b0 = mid ? B[0] : 0.f, c_0 = low ? C[0] : 0.f, d0 = low && mid ? D[0] : 0.f;
-      const double a_r = right ? A[rh] : 0.f, c_r = right && low ? C[rh] : 0.f;
-      const double a_d = down ? A[1] : 0.f, b_d = down && mid ? B[1] : 0.f, a_dr = down && right ? A[rh + 1] : 0.f;
-      const double d_u = up && mid ? D[-1] : 0.f, c_ur = up && right ? C[rh - 1] : 0.f;
+      // rows r0 - 1 .. r0 + 2, columns c0 .. c0 + 2; the next iterate's samples arrive meanwhile
+      double v[11];
+#pragma unroll
+      for (int e = 0; e < 11; e++) v[e] = in_x[e] ? x[t & 1][e] : 0.f;
+      const double a0 = v[0], b0 = v[1], c_0 = v[2], d0 = v[3], a_r = v[4], c_r = v[5], a_d = v[6], b_d = v[7], a_dr = v[8],
+                   d_u = v[9], c_ur = v[10];
+      if (t + 1 < kRcBatch) samples(t + 1, x[(t + 1) & 1]);
       auto px = [](const double (&v)[kRcStencil], double p, double s, double ne, double e, double se) {
         return p * (v[0] * p + 2.0 * (v[1] * s + v[2] * ne + v[3] * e + v[4] * se));
       };

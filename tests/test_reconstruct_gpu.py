@@ -128,3 +128,17 @@ def test_a_long_set_follows_the_interval_chain():
     np.testing.assert_array_equal(g["mask"], o_mask)
     np.testing.assert_allclose(g["data_corrected"][o_mask], o_out[o_mask], rtol=0,
                                atol=1e-4 * np.abs(o_out[o_mask]).max())
+
+
+@pytest.mark.parametrize("dh,dw", [(0, 0), (1, 0), (0, 1), (1, 1)])
+def test_odd_and_even_templates_stop_close_to_the_oracle(dh, dw):
+    """Templates of both parities each way (paired and single stencil loads of the energies, quads that
+    the last row or column cuts): counts within two of the largest check interval."""
+    rec, s, dxk, dyk = _estimated(5, n_frames=4)
+    fr = rec.frames.astype(np.float32)
+    shape = (rec.template.shape[0] - dh, rec.template.shape[1] - dw)
+    g = api.reconstruct_frames(fr, dxk, dyk, s, shape)
+    o_out, o_mask, o_its = _oracle(fr, dxk, dyk, s, shape)
+    np.testing.assert_array_equal(g["mask"], o_mask)
+    its = np.array(g["iterations"])
+    assert np.all(np.abs(its - np.array(o_its)) <= 10 * 2), (its, o_its)
