@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(256) k_rc_coef(RcBufs b, double regfac, double
 // that sweep that far (limit[f] >= it). A colour's eight neighbours are of the other colours: the ones
 // before it come from the new iterate, the ones after it from the old. Neighbours outside the template
 // have zero terms. Bound: HBM, 36 B of terms per pixel (pixel by pixel in memory, 10 floats each, a
-// colour of 64 frames of 512 x 512 took 48 us; colour by colour 42 us, 5.2 TB/s).
+// colour of 64 frames of 512 x 512 took 48 us; colour by colour 41.5 us, 5.2 TB/s).
 template <int COLOUR>
 __global__ void __launch_bounds__(256) k_rc_sweep(RcBufs b, int it, int sold, int snew, const int* __restrict__ limit) {
   const int f = blockIdx.y;
@@ -256,7 +256,8 @@ __global__ void __launch_bounds__(256) k_rc_sweep(RcBufs b, int it, int sold, in
       const int qi = i + ((pr + dr[q] + 2) >> 1) - 1, qj = j + ((pc + dc[q] + 2) >> 1) - 1;
       const bool in = (unsigned)(r + dr[q]) < (unsigned)th && (unsigned)(c + dc[q]) < (unsigned)tw;
       const float* x = (qc < COLOUR ? xn : xo) + qc * nq;
-      v[q] = in ? x[qi + (size_t)rh * qj] : 0.0f;
+      v[q] = x[in ? qi + rh * qj : k];  // (outside: any value of the plane, selected away)
+      if (!in) v[q] = 0.0f;
       t[q] = __ldg(cf + (size_t)q * 4 * nq + k);
     }
     const float L = __ldg(cf + (size_t)8 * 4 * nq + k);
@@ -271,24 +272,27 @@ __global__ void __launch_bounds__(256) k_rc_sweep(RcBufs b, int it, int sold, in
 }
 
 // Linear energy terms of iterates it0 .. it0 + nit - 1 (slots sl.x ..) of the frames that have swept that
-// far: FP32 sums of Le_p x_p, kRcParts CTAs per frame over fixed pixel ranges.
+// far: FP32 sums of Le_p x_p, kRcParts CTAs per frame over fixed pixel ranges. Bound: HBM, 20 B per
+// pixel (four iterates of 64 frames of 512 x 512: 65 us, 5.2 TB/s; 99 with each iterate's load under a
+// branch on nit).
 __global__ void __launch_bounds__(256) k_rc_linear(RcBufs b, int it0, int nit, int4 sl, const int* __restrict__ limit) {
   const int f = blockIdx.y;
   if (limit[f] < it0 + nit - 1) return;
   const int th = b.th, np = b.np;
   const float* le = b.le + (size_t)f * np;
-  const float* xs[kRcBatch] = {rc_iterate(b, sl.x, f), rc_iterate(b, sl.y, f), rc_iterate(b, sl.z, f),
-                               rc_iterate(b, sl.w, f)};
+  // (past the last of nit, the first's again: every load is unconditional)
+  const float* xs[kRcBatch] = {rc_iterate(b, sl.x, f), rc_iterate(b, nit > 1 ? sl.y : sl.x, f),
+                               rc_iterate(b, nit > 2 ? sl.z : sl.x, f), rc_iterate(b, nit > 3 ? sl.w : sl.x, f)};
   const int per = (np + kRcParts - 1) / kRcParts, a = blockIdx.x * per, e = min(np, a + per);
   float ls[kRcBatch] = {};
   int c = (a + (int)threadIdx.x) / th, r = a + (int)threadIdx.x - c * th;
+#pragma unroll 4
   for (int p = a + threadIdx.x; p < e; p += blockDim.x) {
     const int at = ((r & 1) * 2 + (c & 1)) * b.nq + (r >> 1) + b.rh * (c >> 1);  // (4 nq < 2^31)
     const float l = le[p];  // zero at unmasked pixels
     for (r += blockDim.x; r >= th; r -= th) c++;
 #pragma unroll
-    for (int k = 0; k < kRcBatch; k++)
-      if (k < nit) ls[k] = fmaf(l, xs[k][at], ls[k]);
+    for (int k = 0; k < kRcBatch; k++) ls[k] = fmaf(l, xs[k][at], ls[k]);
   }
   __shared__ float sv[kRcBatch][256];
 #pragma unroll
