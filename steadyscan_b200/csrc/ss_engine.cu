@@ -2844,7 +2844,7 @@ int reconstruct_frames(const ss_reconstruct* r) {
   constexpr size_t kRingBytes = size_t(4) << 30;
   const int rh = (th + 1) / 2, cw = (tw + 1) / 2;
   const size_t iterate = 16 * (size_t)rh * cw;  // bytes
-  const int slots = (int)std::min<size_t>(64, std::max<size_t>(kRcBatch + 2, kRingBytes / iterate));
+  const int slots = (int)std::min<size_t>(24, std::max<size_t>(kRcBatch + 2, kRingBytes / iterate));
   const int chunk = (int)std::max<size_t>(1, std::min<size_t>({(size_t)n, (size_t)64, kRingBytes / (iterate * slots)}));
   const size_t px = (size_t)hd * wd, fsz = fr.dtype == SS_F64 ? 8 : 4, osz = o.dtype == SS_F64 ? 8 : 4;
   CallMem m;
