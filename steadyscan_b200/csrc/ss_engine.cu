@@ -942,7 +942,9 @@ struct Batch::Impl {
   cudaEvent_t ev_up = nullptr;
   int* d_ready = nullptr;
   void* early = nullptr;  // streamed frames, their image sums, sum scratch and ready flags (pool)
-  std::vector<std::pair<void*, size_t>> touch;  // more host memory that the run's results go to
+  // Host memory that the run's results go to, of a call that owns it throughout (touch_pages). The outputs
+  // of a batch are the caller's until collect: a run keeps its hands off them.
+  std::vector<std::pair<void*, size_t>> touch;
   bool pool_arena = false;  // the arena comes from the library's memory pool
   // flag t: CUDA-event timing of the stages, summed into the reference's sub-function slots
   // (output 10, timedmainiteration.cpp:45-143 and task.cpp:293-356); the interval from a mark to the
@@ -1937,27 +1939,28 @@ int Batch::poll() {
   return 1;
 }
 
-// The host outputs of a batch whose run has been launched (touch_pages).
+// Adds the host outputs of every group to `touch`: for calls that run and collect in one.
 static void touch_outputs(Batch::Impl* b) {
   for (size_t i = 0; i < b->hg.size(); i++) {
     const HostGroup& g = b->hg[i];
     const size_t nk = (size_t)(g.W + 1) * g.nF * 8;
     if (const ss_outputs* o = b->outs[i]) {
-      touch_pages(o->dx_knots, nk);
-      touch_pages(o->dy_knots, nk);
-      touch_pages(o->mask, (size_t)g.Hb * g.fW);
+      b->touch.emplace_back(o->dx_knots, nk);
+      b->touch.emplace_back(o->dy_knots, nk);
+      b->touch.emplace_back(o->mask, (size_t)g.Hb * g.fW);
     }
   }
-  for (const auto& t : b->touch) touch_pages(t.first, t.second);
 }
 
-int Batch::run() {
+int Batch::run(bool owns_outputs) {
   bool touched = false;
   int rc = start();
   if (rc) return rc;
+  if (owns_outputs) touch_outputs(d);
   for (;;) {
     if ((rc = step())) return rc;
-    if (!touched) touch_outputs(d);
+    if (!touched)
+      for (const auto& t : d->touch) touch_pages(t.first, t.second);
     touched = true;
     SS_CK(cudaStreamSynchronize(d->stream));
     rc = poll();
@@ -3068,7 +3071,7 @@ int ss_align_groups(int32_t n_groups, const ss_inputs* in, ss_outputs* out) {
   ss::Batch b;
   b.set_stream_frames(true);  // frames of later groups upload while earlier groups run
   int rc = b.prepare(n_groups, in, out, nullptr, 0);
-  if (!rc) rc = b.run();
+  if (!rc) rc = b.run(true);
   if (!rc) rc = b.collect();
   if (rc) return rc;
   double ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();

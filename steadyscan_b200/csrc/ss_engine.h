@@ -34,8 +34,10 @@ class Batch {
   // groups already run (each group joins the run when its frames have arrived). For batches run
   // once, such as ss_align_groups; results are those of an unstreamed run.
   void set_stream_frames(bool on);
-  // Runs every group from its initial knots to its stop criterion.
-  int run();
+  // Runs every group from its initial knots to its stop criterion. owns_outputs: the outputs given to
+  // prepare() are this call's until collect() has returned, so their pages are put in place during the
+  // run; otherwise a run does not look at them (the caller may have freed them, or be editing them).
+  int run(bool owns_outputs = false);
   // The same run one cycle at a time without blocking: start() resets every group to its initial
   // knots, step() launches one cycle on the batch stream, poll() returns 0 while that cycle runs,
   // 1 when it has finished and another is needed, 2 when every group has stopped.
