@@ -142,7 +142,9 @@ def _outputs(args: dict, want_mask=True, want_history=False):
     return o, a, (hb, w, nF, N, mi)
 
 
-def _result(o: SSOutputs, a: dict, dims) -> dict:
+def _result(o: SSOutputs, a: dict, dims, own_mask=False) -> dict:
+    """The results in the buffers ``a``, which the caller gives up: the mask is a view of its buffer unless
+    ``own_mask`` (a batch writes the buffer again at its next collect)."""
     hb, w, nF, N, mi = dims
     r = dict(dx=a["dx"], dy=a["dy"], frame_corr=a["frame_corr"], iter_used=int(a["iter_used"][0]),
              residrms=a["residrms"], device_init_time=float(a["device_init_time"][0]),
@@ -152,7 +154,8 @@ def _result(o: SSOutputs, a: dict, dims) -> dict:
              frame_params=a["frame_params"].reshape(nF, 2 * (w + 1), order="F") if "frame_params" in a else None,
              blocks_used=a["blocks_used"].reshape(w, nF, order="F").astype(bool))
     if "mask" in a:
-        r["mask"] = a["mask"].view(np.bool_).reshape(hb, w * nF, order="F")  # 0 / 1 bytes
+        m = a["mask"].astype(bool) if own_mask else a["mask"].view(np.bool_)  # 0 / 1 bytes
+        r["mask"] = m.reshape(hb, w * nF, order="F")
     r["rg_params"] = a["rg_params"].reshape(2 * N, 2 * mi, order="F") if "rg_params" in a else None
     r["function_times"] = a.get("function_times")
     r["iteration_times"] = a.get("iteration_times")
@@ -497,7 +500,7 @@ class Batch:
 
     def collect(self) -> list:
         check(self._lib.ss_batch_collect(self._h))
-        return [_result(self._outs[k], self._arrays[k], self._dims[k]) for k in range(len(self._dims))]
+        return [_result(self._outs[k], self._arrays[k], self._dims[k], own_mask=True) for k in range(len(self._dims))]
 
     def set_timing(self, on: bool):
         check(self._lib.ss_batch_set_timing(self._h, 1 if on else 0))

@@ -54,3 +54,17 @@ def test_a_run_leaves_the_outputs_alone():
     np.testing.assert_array_equal(got.astype(bool), ref["mask"])
     for k in ("dx", "dy"):
         np.testing.assert_array_equal(np.frombuffer(pages[k + "_knots"].m, np.float64, ref[k].size), ref[k])
+
+
+def test_a_mask_outlives_the_next_collect():
+    args, _, _ = make_args(nlines=32, linewidth=32, nknots=9, n_frames=4, settings={"max_iter": 4})
+    b = api.Batch([args], want_mask=True)
+    b.run()
+    first = b.collect()[0]["mask"]
+    ref = first.copy()
+    assert ref.any()
+    first[:] = False  # the caller's own
+    b.run()
+    second = b.collect()[0]["mask"]
+    np.testing.assert_array_equal(second, ref)
+    assert not first.any() and second.flags.f_contiguous
