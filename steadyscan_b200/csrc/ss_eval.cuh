@@ -540,7 +540,8 @@ __device__ __forceinline__ void trial_column(const GroupDesc& G, size_t coli, co
 
 // Assembly sums of one block column with one warp (FP64), the mask and difference-image knots the same
 // and every block column's tfrac the same: eval_column<kAssemble>'s arithmetic, two rows of a lane's step
-// at a time (the recording above: 4.8 -> 3.3 ms of assembly a run). Its SSD adds in trial_column's order: a trial that moves no knot gives the same sum.
+// at a time (400 frames of 256 x 512 FP64, knots every 4 lines: 4.8 -> 3.3 ms of assembly a run). Its SSD
+// adds in the order of trial_column of the same RUN, eval_column's in the order of RUN 1.
 template <class FrameT, int RUN>
 __device__ __forceinline__ void assemble_column(const GroupDesc& G, size_t coli, const ColGeo<double>& geo,
                                                 const ColKnots<double>& k, double (&out)[kCsStride], int& cnt_out) {
@@ -987,7 +988,10 @@ __global__ void __launch_bounds__(kLsThreads, SS_LS_BLOCKS)
     return geo;
   };
   if (threadIdx.x == 0) atomicAdd(G.staging + 2, 1ull);
-  const bool run4 = run4_ok<FrameT>(G);
+  // A trial's column sums add in the order of the assembly's, so that a trial that moves no knot is no
+  // improvement: runs of 4 rows where assemble_column takes them (the assembled columns of a searching frame
+  // are never dual), single rows where eval_column assembles (tfrac differs between block columns).
+  const bool run4 = run4_ok<FrameT>(G), trial4 = run4 && G.frac_uniform;
   const double thr = G.move_thresh, rho = G.ls_mult;
   int trials = 0;
   while (searching) {
@@ -1003,7 +1007,7 @@ __global__ void __launch_bounds__(kLsThreads, SS_LS_BLOCKS)
       double qs;
       int qc;
       const size_t coli = (size_t)(b0 + t) * Hb;
-      if (run4) trial_column<FrameT, 4>(G, coli, column_geo(t), x0, x1, y0, y1, qs, qc);
+      if (trial4) trial_column<FrameT, 4>(G, coli, column_geo(t), x0, x1, y0, y1, qs, qc);
       else trial_column<FrameT, 1>(G, coli, column_geo(t), x0, x1, y0, y1, qs, qc);
       ssd += qs;
       cnt += qc;
