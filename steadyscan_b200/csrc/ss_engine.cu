@@ -2523,9 +2523,19 @@ struct CallMem {
       if (!(pool = work_pool(dev))) return nullptr;
     }
     void* q = nullptr;
-    if (cudaMallocFromPoolAsync(&q, std::max<size_t>(1, count) * sizeof(T), pool, s) != cudaSuccess) return nullptr;
+    if (cudaMallocFromPoolAsync(&q, std::max<size_t>(1, count) * sizeof(T), pool, s) != cudaSuccess) {
+      cudaGetLastError();  // reported by the caller, not by the next launch check
+      return nullptr;
+    }
     ptrs.push_back(q);
     return static_cast<T*>(q);
+  }
+  // Frees what was taken after the first `keep` and gives the pool's idle memory back to the device.
+  void release(size_t keep) {
+    for (size_t i = keep; i < ptrs.size(); i++) cudaFreeAsync(ptrs[i], s);
+    ptrs.resize(std::min(keep, ptrs.size()));
+    cudaStreamSynchronize(s);
+    if (pool) cudaMemPoolTrimTo(pool, 0);
   }
 };
 
@@ -2841,14 +2851,17 @@ int reconstruct_frames(const ss_reconstruct* r) {
   if (r->gpu_device_id < 0 || r->gpu_device_id >= ndev) return fail(SS_ERR_INVALID_ARGUMENT, "gpu_device_id out of range");
   SS_CK(cudaSetDevice(r->gpu_device_id));
 
-  // Iterates kept per frame (slot 0, the first guess, and a ring of the later ones): 64 where 64 frames of
-  // them fit in kRingBytes (a 512 x 512 frame takes 64 MB), so that a set's outputs are at hand when its
-  // stops are known; larger frames run fewer at a time, and the largest with a shorter ring.
+  // Iterates kept per frame: slot 0, the first guess, and a ring of the later ones, so that a set's outputs are
+  // at hand when its stops are known (an iterate that the ring has lost is swept again from the first guess).
+  // 24, so that 64 frames of up to 836 x 836 run together in kRingBytes; larger frames run fewer at a time,
+  // and the largest with a shorter ring. Where the device has less memory left, the ring is cut to the
+  // shortest, then the frames of a part are halved.
   constexpr size_t kRingBytes = size_t(4) << 30;
+  constexpr int kMinSlots = kRcBatch + 2;
   const int rh = (th + 1) / 2, cw = (tw + 1) / 2;
   const size_t iterate = 16 * (size_t)rh * cw;  // bytes
-  const int slots = (int)std::min<size_t>(24, std::max<size_t>(kRcBatch + 2, kRingBytes / iterate));
-  const int chunk = (int)std::max<size_t>(1, std::min<size_t>({(size_t)n, (size_t)64, kRingBytes / (iterate * slots)}));
+  int slots = (int)std::min<size_t>(24, std::max<size_t>(kMinSlots, kRingBytes / iterate));
+  int chunk = (int)std::max<size_t>(1, std::min<size_t>({(size_t)n, (size_t)64, kRingBytes / (iterate * slots)}));
   const size_t px = (size_t)hd * wd, fsz = fr.dtype == SS_F64 ? 8 : 4, osz = o.dtype == SS_F64 ? 8 : 4;
   CallMem m;
   m.dev = r->gpu_device_id;
@@ -2876,31 +2889,47 @@ int reconstruct_frames(const ss_reconstruct* r) {
   b.rh = rh;
   b.cw = cw;
   b.nq = rh * cw;
-  b.frames = chunk;
-  const size_t cnp = (size_t)chunk * np;
-  b.wy = m.take<double>(cnp);
-  b.ww = m.take<double>(cnp * kRcStencil);
-  b.z = m.take<float>(cnp);
-  b.cnt = m.take<float>(cnp);
-  b.last_z = m.take<int>(cnp);
-  b.last_n = m.take<int>(cnp);
-  b.mask = m.take<uint8_t>(cnp);
-  b.coef = m.take<float>((size_t)chunk * kRcTerms * 4 * b.nq);
-  b.le = m.take<float>(cnp);
-  b.x = m.take<float>((size_t)slots * chunk * 4 * b.nq);
-  b.part = m.take<double>((size_t)chunk * kRcParts * kRcBatch);
-  b.part_l = m.take<float>((size_t)chunk * kRcParts * kRcBatch);
-  int* d_limit = m.take<int>(chunk);
-  int* d_count = m.take<int>(chunk);
-  int* d_skip = m.take<int>(chunk);
-  int* d_slot = m.take<int>(chunk);
-  float* d_energy = m.take<float>((size_t)chunk * kRcBatch);
-  void* d_out = o.location == SS_DEVICE ? const_cast<void*>(o.data) : m.take<char>(osz * cnp);
-  uint8_t* d_mk = r->mask ? m.take<uint8_t>(cnp) : nullptr;
-  if (!d_bx || !d_by || !d_tf || !d_pk || !d_dxk || !d_dyk || !d_data || !b.wy || !b.ww || !b.z || !b.cnt ||
-      !b.last_z || !b.last_n || !b.mask || !b.coef || !b.le || !b.x || !b.part || !b.part_l || !d_limit || !d_count ||
-      !d_skip || !d_slot || !d_energy || !d_out || (r->mask && !d_mk))
+  int *d_limit = nullptr, *d_count = nullptr, *d_skip = nullptr, *d_slot = nullptr;
+  float* d_energy = nullptr;
+  void* d_out = nullptr;
+  uint8_t* d_mk = nullptr;
+  auto work_memory = [&]() -> bool {  // of a part of `chunk` frames with `slots` iterates
+    b.frames = chunk;
+    const size_t cnp = (size_t)chunk * np;
+    b.wy = m.take<double>(cnp);
+    b.ww = m.take<double>(cnp * kRcStencil);
+    b.mask = m.take<uint8_t>(cnp);
+    b.coef = m.take<float>((size_t)chunk * kRcTerms * 4 * b.nq);
+    b.le = m.take<float>(cnp);
+    b.x = m.take<float>((size_t)slots * chunk * 4 * b.nq);
+    b.part = m.take<double>((size_t)chunk * kRcParts * kRcBatch);
+    b.part_l = m.take<float>((size_t)chunk * kRcParts * kRcBatch);
+    d_limit = m.take<int>(chunk);
+    d_count = m.take<int>(chunk);
+    d_skip = m.take<int>(chunk);
+    d_slot = m.take<int>(chunk);
+    d_energy = m.take<float>((size_t)chunk * kRcBatch);
+    d_out = o.location == SS_DEVICE ? const_cast<void*>(o.data) : m.take<char>(osz * cnp);
+    d_mk = r->mask ? m.take<uint8_t>(cnp) : nullptr;
+    if (!b.wy || !b.ww || !b.mask || !b.coef || !b.le || !b.x || !b.part || !b.part_l || !d_limit || !d_count ||
+        !d_skip || !d_slot || !d_energy || !d_out || (r->mask && !d_mk))
+      return false;
+    // the first guess's sums lie where the sweep terms are written once it stands
+    static_assert(kRcTerms * 4 >= 4 * 4, "four planes of np in the terms' quarter planes (4 nq >= np)");
+    b.z = b.coef;
+    b.cnt = b.coef + cnp;
+    b.last_z = reinterpret_cast<int*>(b.coef + 2 * cnp);
+    b.last_n = reinterpret_cast<int*>(b.coef + 3 * cnp);
+    return true;
+  };
+  if (!d_bx || !d_by || !d_tf || !d_pk || !d_dxk || !d_dyk || !d_data)
     return fail(SS_ERR_OUT_OF_MEMORY, "reconstruct: work memory");
+  for (const size_t kept = m.ptrs.size(); !work_memory();) {
+    m.release(kept);
+    if (slots > kMinSlots) slots = kMinSlots;
+    else if (chunk > 1) chunk = (chunk + 1) / 2;
+    else return fail(SS_ERR_OUT_OF_MEMORY, "reconstruct: work memory");
+  }
   SS_CK(cudaMemcpyAsync(d_bx, bx.data(), px * 8, cudaMemcpyHostToDevice, s));
   SS_CK(cudaMemcpyAsync(d_by, by.data(), px * 8, cudaMemcpyHostToDevice, s));
   SS_CK(cudaMemcpyAsync(d_tf, tf.data(), px * 8, cudaMemcpyHostToDevice, s));

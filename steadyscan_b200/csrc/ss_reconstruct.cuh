@@ -50,12 +50,12 @@ struct RcBufs {
   int frames;       // frames of a slot
   double* wy;       // np
   double* ww;       // kRcStencil planes of np
-  float* z;         // np: push-grid sums, then the first guess
+  float* z;         // np: push-grid sums
   float* cnt;       // np: push-grid weights
   int* last_z;      // np
   int* last_n;      // np
   uint8_t* mask;    // np
-  float* coef;      // kRcTerms x 4 quarter planes
+  float* coef;      // kRcTerms x 4 quarter planes (before them z, cnt, last_z and last_n)
   float* le;        // np: single(Lfull) of masked pixels, else 0
   float* x;         // [slot][frame] iterates of 4 quarter planes; slot 0 is the first guess
   double* part;     // frames x kRcParts x kRcBatch: energy partial sums (FP64 quadratic, FP32 linear)
