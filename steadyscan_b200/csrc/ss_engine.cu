@@ -2600,7 +2600,7 @@ static int row_blocks(const int* gather, int hb, int nb, int hc, int wc, std::ve
     if (k > kRowMaxLines || (int64_t)k * wc > hb) return 0;
     const int m = k * wc;
     int bad = 0;
-    for (int r = k; r < m; r++) bad |= (g[r] - g[r - k]) ^ hc;
+    for (int r = k; r < m; r++) bad |= (int)((unsigned)g[r] - (unsigned)g[r - k]) ^ hc;
     for (int r = m; r < hb; r++) bad |= g[r] ^ -1;
     if (bad) return 0;
     start[b] = s;
@@ -2669,8 +2669,9 @@ int prepare_frames(const ss_prep_frames* p) {
   const int hb = p->block_h, nbk = p->n_blocks;
   if (!p->gather || hb < 1 || nbk < 1) return fail(SS_ERR_INVALID_ARGUMENT, "prepare_frames: empty block map");
   BlockMap map;
-  // the tiles' frame index is the grid's z extent and the column tiles its y extent
-  if (hc <= INT_MAX && wc <= (int64_t)65535 * kRowTile)
+  // the tiles' frame index is the grid's z extent and the column tiles its y extent; a map of a larger frame
+  // cannot name every pixel (its entries would wrap)
+  if (hc * wc <= INT_MAX && wc <= (int64_t)65535 * kRowTile)
     map.kmax = row_blocks(p->gather, hb, nbk, (int)hc, (int)wc, map.start);
   if (!map.kmax) {
     int lo = 0;
