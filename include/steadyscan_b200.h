@@ -172,6 +172,8 @@ typedef struct ss_batch_stats {
 
 SS_API int ss_batch_create(int32_t n_groups, const ss_inputs* in, ss_outputs* out, ss_batch** batch);
 SS_API int ss_batch_run(ss_batch* batch);
+/* Writes the outputs. They are the caller's until then: a run neither reads nor writes their buffers, and
+ * takes the addresses that the ss_outputs hold when it is collected. */
 SS_API int ss_batch_collect(ss_batch* batch);
 /* 1 turns on CUDA-event timing of the evaluation kernels for later runs (adds events to the stream). */
 SS_API int ss_batch_set_timing(ss_batch* batch, int32_t on);
@@ -252,11 +254,11 @@ SS_API int ss_solve_block_tridiagonal(int32_t n, const double* diag, const doubl
  * ss_solve_block_tridiagonal; the workspace is a fixed device array inside this library of
  * 32768 blocks (3.4 MB, held by every GPU that loads the library until the process exits), so
  * n > 32768 is rejected with SS_ERR_INVALID_ARGUMENT. The first call on a device looks up that
- * array's device address (again after the device's context has been reset, e.g. by cudaDeviceReset). Each call waits for `stream`
- * (cudaStreamSynchronize) before it returns. All calls
- * share the one array per device: calls that overlap on the GPU (different streams or threads at
- * the same time) race and corrupt each other's results; serialize them. Each call writes every part
- * of the workspace it reads before reading it. */
+ * array's device address (again after the device's context has been reset, e.g. by
+ * cudaDeviceReset). Each call waits for `stream` (cudaStreamSynchronize) before it returns. All
+ * calls share the one array per device: calls that overlap on the GPU (different streams or threads
+ * at the same time) race and corrupt each other's results; serialize them. Each call writes every
+ * part of the workspace it reads before reading it. */
 SS_API int ss_solve_block_tridiagonal_noalloc(int32_t n, const double* diag, const double* coupling,
                                               const double* rhs, double* x, void* stream);
 

@@ -171,8 +171,8 @@ struct Sample {
 
 // Bilinear template value and warped gradients at a valid pixel (task_differenceimage.cuh:118-126,
 // task_updategradients.cu:12-20). FP64 templates are rows, whose corners neighbouring lanes share in
-// L1; a 32-byte quad per pixel made the FP64 passes L2-bound. With gquad == nullptr the gradients are the template's forward
-// differences (steady_scan.m:178-179), taken from the same four template values.
+// L1; a 32-byte quad per pixel made the FP64 passes L2-bound. With gquad == nullptr the gradients are
+// the template's forward differences (steady_scan.m:178-179), taken from the same four template values.
 template <class Acc, class TplT, bool kGrad>
 __device__ __forceinline__ Sample<Acc> sample(const GroupDesc& G, Acc x, Acc y) {
   Acc xf, yf;

@@ -11,9 +11,9 @@
 // weights fall below 1e-20 of the centre tap: the terms left out lie below FP64 rounding of the sum.
 // Median normalisation divides each (blurred) frame by the median of its H x W samples, found
 // exactly by narrowing a range of order-preserving 64-bit keys (NaN anywhere gives NaN, as MATLAB's
-// median); the division happens as the samples are put in block order. Block reorder: entry (r, b) of a frame's block matrix is the cropped frame's pixel whose
-// column-major index the caller's gather map holds there, or 0 where it holds -1
-// (image2blockmatrix, steady_scan.m:601-613).
+// median); the division happens as the samples are put in block order. Block reorder: entry (r, b) of
+// a frame's block matrix is the cropped frame's pixel whose column-major index the caller's gather map
+// holds there, or 0 where it holds -1 (image2blockmatrix, steady_scan.m:601-613).
 #pragma once
 
 #include <cooperative_groups.h>
@@ -67,10 +67,11 @@ __global__ void __launch_bounds__(256) k_blur_pass(const void* __restrict__ in, 
 }
 
 // The tiled blur passes. Bound: the FP64 pipe (2 R + 1 operations per output and pass). A thread
-// computes Q neighbouring outputs from two windows of Q samples that slide outwards one tap at a time, so a tap costs it two shared-memory loads and 2 Q FP64 operations in place of 2 Q
-// cached global loads: 256 frames of 512 x 512 uint16, R = 10: the two passes 1240 us by
-// k_blur_pass, 660 us here (the FP64 pipe 20-30% busy: staging and index work share the issue slots). Down a column the count is odd: lanes that many samples apart read different
-// banks.
+// computes Q neighbouring outputs from two windows of Q samples that slide outwards one tap at a time,
+// so a tap costs it two shared-memory loads and 2 Q FP64 operations in place of 2 Q cached global loads:
+// 256 frames of 512 x 512 uint16, R = 10: the two passes 1240 us by k_blur_pass, 743 us here (the
+// FP64 pipe 20-30% busy: staging and index work share the issue slots). Down a column the count is odd:
+// lanes that many samples apart read different banks.
 constexpr int kBlurDown = 9, kBlurAlong = 8;  // outputs of a thread: down the columns, along the rows
 constexpr int kBlurMaxR = 320;  // the row pass stages (64 + 2 R) x 32 doubles in shared memory
 constexpr int kBlurSeg = 32 * kBlurDown;    // outputs of a warp down a column
@@ -205,7 +206,7 @@ struct KeyRange {
   }
 };
 
-// Along the rows; lanes on 32 consecutive lines, a warp per kBlurOut columns. With stats, also each
+// Along the rows; lanes on 32 consecutive lines, a warp per kBlurAlong columns. With stats, also each
 // frame's key range. Grid: (ceil(h / 32), ceil(w / kBlurCols), frames).
 __global__ void __launch_bounds__(256) k_blur_rows(const double* __restrict__ in, double* __restrict__ out, int h, int w,
                                                    int period, const double* __restrict__ taps, int R,
@@ -481,8 +482,7 @@ __global__ void __launch_bounds__(256) k_block_gather(const void* __restrict__ i
 // starts at word j * pitch + j / 4: the 4 columns of a thread's 8 entries (2 lines per block) then
 // fall into different banks across the warp. K > 0: every block has K lines and the index arithmetic
 // is shifts and constants (the default scan's 1, 2 and 4 lines per knot). With med, every sample is
-// divided by its frame's median. Grid: (block tiles, column
-// tiles, frames).
+// divided by its frame's median. Grid: (block tiles, column tiles, frames).
 constexpr int kRowTile = 64;
 constexpr int kRowMaxLines = 32;  // longer runs are coalesced already in k_block_gather
 template <class InT, class OutT, int VE, int VO, int K>

@@ -11,8 +11,8 @@ constexpr int kCrStride = 13;  // D(3: xx yy xy) L(4) R(4) b(2)
 
 // The CTAs of a solve cluster: a chain is solved by up to kSolveCluster CTAs that hold its separator
 // system in their shared memory together. One 1024-thread CTA per chain was bound by that SM's memory
-// queue (16385 knots: 158 us per half-step solve; ss_solve_block_tridiagonal of 16385 blocks 670 us
-// with its allocation, now 68 us).
+// queue (16385 knots: 158 us per half-step solve; a call of ss_solve_block_tridiagonal of 16385 blocks
+// 693 us with its allocation, now 85 us).
 constexpr int kSolveCluster = 8;
 constexpr int kSolveSysThreads = kSolveThreads / kSolveCluster;  // a partition per thread of the cluster
 

@@ -28,8 +28,8 @@
 // as its own iterate (in a ring of slots) with its energy, and the host follows the chain of intervals
 // over the energies; a frame sweeps until its stop is known, or the stop of every interval 1..10 is.
 // Guessing the intervals and sweeping again from the first wrong guess took seven runs of a 64-frame
-// set and a separate copy of every kept iterate (64 frames of 512 x 512: 150 ms a call, 119 of them on
-// the device; here 44 and 20).
+// set and a separate copy of every kept iterate (64 frames of 512 x 512: 153 ms a call, 119 of them on
+// the device; here 37 and 20).
 #pragma once
 
 #include "ss_common.cuh"
@@ -149,10 +149,6 @@ __global__ void __launch_bounds__(256) k_rc_pushgrid(RcBufs b, const void* __res
       if (ln[tn] == q) b.cnt[(size_t)f * b.np + tn] += (float)wc[cn];
     }
   }
-}
-
-__global__ void k_rc_fill_int(int* p, size_t n, int v) {
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) p[e] = v;
 }
 
 // Stencil plane of the pair (p, p + th - 1): NE, or S where the template has two rows and the offsets

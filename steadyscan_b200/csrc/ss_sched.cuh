@@ -1,9 +1,9 @@
 // Tile schedules of the evaluation launches.
 //
 // An evaluation tile is one block column of one chunk of G.frames_per_cta consecutive frames of a
-// group. Before each evaluation launch one CTA of k_schedule lists the (group, frame chunk) entries
-// that have work in that launch (the group's phase for the mode; for a trial round, a frame of the
-// chunk still searching), each standing for the group's W tiles, with the prefix sum of their tiles.
+// group. Before each evaluation launch one CTA lists the (group, frame chunk) entries that have work in
+// that launch (the group's phase for the mode), each standing for the group's W tiles, with the prefix
+// sum of their tiles; trial rounds list the frames still searching (build_trial_schedule below).
 // The evaluation kernels then run as a grid of resident CTAs that take tiles from the list through
 // an atomic counter, so a launch costs in proportion to the work left, not to the batch's size:
 // late trial rounds of a ragged batch, where a few long searches remain, launch no idle CTAs.
@@ -58,13 +58,7 @@ __device__ __forceinline__ int build_schedule(const GroupDesc* __restrict__ gds,
       g = chunk_group[j];
       const GroupDesc& G = gds[g];
       fb = j - G.chunk_base;
-      bool on = group_has_work<MODE>(ctl[g]);
-      if (on && MODE == kTrial) {
-        const int f0 = fb * G.frames_per_cta, f1 = min(G.nF, f0 + G.frames_per_cta);
-        on = false;
-        for (int f = f0; f < f1 && !on; f++) on = (G.fstate[f] & 2) != 0;
-      }
-      w = on ? G.W : 0;
+      w = group_has_work<MODE>(ctl[g]) ? G.W : 0;
     }
     // exclusive scans of the entries and their tiles over the CTA
     const unsigned bal = __ballot_sync(0xffffffffu, w > 0);
