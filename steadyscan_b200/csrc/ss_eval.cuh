@@ -538,11 +538,12 @@ __device__ __forceinline__ void trial_column(const GroupDesc& G, size_t coli, co
   cnt = warp_sum(c);
 }
 
-// Assembly sums of one block column with one warp (FP64), the mask and difference-image knots the same
-// and every block column's tfrac the same: eval_column<kAssemble>'s arithmetic, two rows of a lane's step
-// at a time (400 frames of 256 x 512 FP64, knots every 4 lines: 4.8 -> 3.3 ms of assembly a run). Its SSD
-// adds in the order of trial_column of the same RUN, eval_column's in the order of RUN 1.
-template <class FrameT, int RUN>
+// Assembly sums of one block column with one warp (FP64), the mask and difference-image knots the same:
+// eval_column<kAssemble>'s arithmetic, two rows of a lane's step at a time (400 frames of 256 x 512 FP64,
+// knots every 4 lines: 4.8 -> 3.3 ms of assembly a run). NEXT: the next block column's tfrac differs from
+// this one's. The SSD adds in the order of trial_column of the same RUN, eval_column's in that of RUN 1: a
+// trial that moves no knot gives the same column sums wherever eval_tile takes the search's RUN.
+template <class FrameT, int RUN, bool NEXT>
 __device__ __forceinline__ void assemble_column(const GroupDesc& G, size_t coli, const ColGeo<double>& geo,
                                                 const ColKnots<double>& k, double (&out)[kCsStride], int& cnt_out) {
   const int Hb = G.Hb;
@@ -551,10 +552,11 @@ __device__ __forceinline__ void assemble_column(const GroupDesc& G, size_t coli,
   int cnt = 0;
 #pragma unroll 1
   for (int r0 = 0; r0 < Hb; r0 += 32 * kStep) {
-    double img[kStep], fr[kStep], bx[kStep];
+    double img[kStep], fr[kStep], bx[kStep], fn[kStep];
     step_frame<RUN, FrameT>(G.image, coli, r0, Hb, img);
     step_doubles<RUN>(geo.frac, r0, Hb, fr);
     step_doubles<RUN>(geo.bx, r0, Hb, bx);
+    if (NEXT) step_doubles<RUN>(geo.fnext, r0, Hb, fn);
 #pragma unroll
     for (int h = 0; h < kStep; h += 2) {
       Sample<double> sa[2];
@@ -573,15 +575,15 @@ __device__ __forceinline__ void assemble_column(const GroupDesc& G, size_t coli,
         cnt += m[e] ? 1 : 0;
         const double f = fr[h + e];
         const double wx = m[e] ? sa[e].wx : 0.0, wy = m[e] ? sa[e].wy : 0.0, d = m[e] ? img[h + e] - sa[e].wI : 0.0;
-        const double fsq = f * f, csq = (1.0 - f) * (1.0 - f), fc = f - fsq;
+        const double fsq = f * f, csq = (1.0 - f) * (1.0 - f), fc = f - fsq, fnsq = NEXT ? fn[h + e] * fn[h + e] : fsq;
         const double gxx = wx * wx, gyy = wy * wy, gxy = wx * wy;
         s[kCsSsd] = fma(d, d, s[kCsSsd]);
         s[kCsAxx] = fma(gxx, csq, s[kCsAxx]);
         s[kCsAyy] = fma(gyy, csq, s[kCsAyy]);
         s[kCsAxy] = fma(gxy, csq, s[kCsAxy]);
-        s[kCsBxx] = fma(gxx, fsq, s[kCsBxx]);
-        s[kCsByy] = fma(gyy, fsq, s[kCsByy]);
-        s[kCsBxy] = fma(gxy, fsq, s[kCsBxy]);
+        s[kCsBxx] = fma(gxx, fnsq, s[kCsBxx]);
+        s[kCsByy] = fma(gyy, fnsq, s[kCsByy]);
+        s[kCsBxy] = fma(gxy, fnsq, s[kCsBxy]);
         s[kCsOxx] = fma(gxx, fc, s[kCsOxx]);
         s[kCsOyy] = fma(gyy, fc, s[kCsOyy]);
         s[kCsOxy] = fma(gxy, fc, s[kCsOxy]);
@@ -858,10 +860,11 @@ __device__ __forceinline__ void eval_tile(const GroupDesc& G, const GroupCtl& C,
         if (affine) eval_column<Acc, FrameT, TplT, MODE, true>(G, coli, geo, k, out, cnt, mo, cc);
         else eval_column<Acc, FrameT, TplT, MODE>(G, coli, geo, k, out, cnt, mo);
       }
-    } else if (MODE == kAssemble && G.frac_uniform && !k.dual) {
+    } else if (MODE == kAssemble && (G.frac_uniform || run4) && !k.dual) {
       if constexpr (sizeof(Acc) == 8) {
-        if (run4) assemble_column<FrameT, 4>(G, coli, geo, k, out, cnt);
-        else assemble_column<FrameT, 1>(G, coli, geo, k, out, cnt);
+        if (!run4) assemble_column<FrameT, 1, false>(G, coli, geo, k, out, cnt);
+        else if (G.frac_uniform) assemble_column<FrameT, 4, false>(G, coli, geo, k, out, cnt);
+        else assemble_column<FrameT, 4, true>(G, coli, geo, k, out, cnt);
       }
     } else if (MODE != kAssemble && !k.dual) {
       if constexpr (sizeof(Acc) == 8) {
@@ -988,10 +991,9 @@ __global__ void __launch_bounds__(kLsThreads, SS_LS_BLOCKS)
     return geo;
   };
   if (threadIdx.x == 0) atomicAdd(G.staging + 2, 1ull);
-  // A trial's column sums add in the order of the assembly's, so that a trial that moves no knot is no
-  // improvement: runs of 4 rows where assemble_column takes them (the assembled columns of a searching frame
-  // are never dual), single rows where eval_column assembles (tfrac differs between block columns).
-  const bool run4 = run4_ok<FrameT>(G), trial4 = run4 && G.frac_uniform;
+  // A trial's column sums add in the order of the assembly's (eval_tile), so that a trial that moves no knot
+  // is no improvement.
+  const bool run4 = run4_ok<FrameT>(G);
   const double thr = G.move_thresh, rho = G.ls_mult;
   int trials = 0;
   while (searching) {
@@ -1007,7 +1009,7 @@ __global__ void __launch_bounds__(kLsThreads, SS_LS_BLOCKS)
       double qs;
       int qc;
       const size_t coli = (size_t)(b0 + t) * Hb;
-      if (trial4) trial_column<FrameT, 4>(G, coli, column_geo(t), x0, x1, y0, y1, qs, qc);
+      if (run4) trial_column<FrameT, 4>(G, coli, column_geo(t), x0, x1, y0, y1, qs, qc);
       else trial_column<FrameT, 1>(G, coli, column_geo(t), x0, x1, y0, y1, qs, qc);
       ssd += qs;
       cnt += qc;
