@@ -811,6 +811,9 @@ __device__ __forceinline__ void eval_tile(const GroupDesc& G, const GroupCtl& C,
     if (win.p) atomicAdd(G.staging + 1, 1ull);
   }
   const bool run4 = sizeof(Acc) == 8 && run4_ok<FrameT>(G);
+  // form of assemble_column: 0 none (eval_column), 1 single rows, 2 runs of 4, 3 those with the next column's
+  // tfrac (one test per frame: with the group's flag read again at each, 4% more of a 256 x 256 assembly)
+  const int form = MODE != kAssemble || sizeof(Acc) != 8 ? 0 : run4 ? (G.frac_uniform ? 2 : 3) : G.frac_uniform ? 1 : 0;
   for (int f = fb * fpc + warp; f < f_end; f += kEvalWarps) {
     const int c = f * W + cc;
     ColKnots<Acc> k;
@@ -860,10 +863,10 @@ __device__ __forceinline__ void eval_tile(const GroupDesc& G, const GroupCtl& C,
         if (affine) eval_column<Acc, FrameT, TplT, MODE, true>(G, coli, geo, k, out, cnt, mo, cc);
         else eval_column<Acc, FrameT, TplT, MODE>(G, coli, geo, k, out, cnt, mo);
       }
-    } else if (MODE == kAssemble && (G.frac_uniform || run4) && !k.dual) {
+    } else if (MODE == kAssemble && form != 0 && !k.dual) {
       if constexpr (sizeof(Acc) == 8) {
-        if (!run4) assemble_column<FrameT, 1, false>(G, coli, geo, k, out, cnt);
-        else if (G.frac_uniform) assemble_column<FrameT, 4, false>(G, coli, geo, k, out, cnt);
+        if (form == 2) assemble_column<FrameT, 4, false>(G, coli, geo, k, out, cnt);
+        else if (form == 1) assemble_column<FrameT, 1, false>(G, coli, geo, k, out, cnt);
         else assemble_column<FrameT, 4, true>(G, coli, geo, k, out, cnt);
       }
     } else if (MODE != kAssemble && !k.dual) {
